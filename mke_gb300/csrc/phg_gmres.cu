@@ -29,14 +29,16 @@
 // multigrid descriptor is read from device memory through a pointer.
 //
 // Every wait is bounded: a barrier that spins longer than ~1 s (clock64)
-// raises a device error flag; all blocks see the flag at their next barrier
-// and return, and the host reports status 2.
+// raises the launch's error flag and poisons its group's arrival count; the
+// group's blocks see the poison at their next barrier and return (groups wait
+// on nothing of one another), and the host reports status 2.
 #include <cmath>
 #include <cstdio>
 #include <mutex>
 
 #include <cooperative_groups.h>
 
+#include "phg_group.cuh"
 #include "phg_kernels.cuh"
 
 namespace phg {
@@ -45,11 +47,9 @@ namespace cg = cooperative_groups;
 
 namespace {
 
-constexpr int MAXM = 48;         // largest restart length
 constexpr int BLOCK = 256;
 constexpr int NWARP = BLOCK / 32;
 constexpr double INNER_RTOL = 1e-5;  // FP32 cycle: reduce the residual 1e5x, then refine
-constexpr long long SPIN_LIMIT = 2000000000LL;  // default wait limit, clock64 cycles (~1 s)
 constexpr int CHEB_KMAX = 64;    // most Chebyshev steps per refinement cycle
 constexpr int LS_MIN_RHS = 32;   // right-hand sides from which the lockstep path runs
 constexpr int LS_MIN_TUNED = 8;  // the fewest for which the autotuner may choose it
@@ -118,89 +118,6 @@ struct Params {
     MultiSeg seg[MAXSEG];
 };
 
-// phase cycle counters kept by block 0 when PHG_PHASE_TIMING is set
-enum { T_RESID, T_VCYCLE, T_SPMV_DOT, T_DOT_SUM, T_UPDATE, T_NORM_SUM, T_GIVENS, T_CORR, T_BARRIER,
-       T_BARRIERS, T_TOTAL, T_NPHASE };
-
-__device__ __forceinline__ int ld_volatile(const int *p) { return *(const volatile int *)p; }
-
-// Barrier over the G blocks of one group; false if the grid is aborting.
-__device__ __forceinline__ unsigned long long ld_acquire(const unsigned long long *p) {
-    unsigned long long v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-
-// The launch's barrier wait limit, held by thread 0 of every block (the only
-// thread that waits): set once at kernel entry from Params::wait_limit.
-__device__ __forceinline__ long long &wait_limit_slot() {
-    __shared__ long long lim;
-    return lim;
-}
-
-// Barriers this block has passed in the launch, held by thread 0 (set to 0 at
-// kernel entry, with the wait limit).
-__device__ __forceinline__ unsigned long long &bar_epoch() {
-    __shared__ unsigned long long e;
-    return e;
-}
-
-// Barrier of the G blocks of one group.  The group's 64-bit word at bar
-// counts arrivals and is never reset within a launch (nor wraps).  Every
-// block of a group passes the same sequence of barriers, so at its k-th
-// barrier (k from 1) a block adds one and waits until the count reaches
-// k * G: the last arrival releases everyone (no reset, no second flag), and a
-// block that runs ahead into the next barrier only raises the count further.
-// The arrival is a release reduction that returns nothing: the block starts
-// polling at once instead of waiting a round trip to L2 for an atomic's old
-// value.  The wait gives up after the launch's wait limit (wait_limit_slot,
-// SPIN_LIMIT by default) and raises the launch's error flag.
-__device__ bool group_sync(unsigned *bar, int G, int *err, long long *tm) {
-    __shared__ int ok;
-    long long tb = (tm && threadIdx.x == 0) ? clock64() : 0;
-    __syncthreads();
-    if (G == 1) {
-        if (tm && threadIdx.x == 0) { tm[T_BARRIER] += clock64() - tb; tm[T_BARRIERS]++; }
-        return ld_volatile(err) == 0;
-    }
-    if (threadIdx.x == 0) {
-        ok = 1;
-        unsigned long long *cnt = reinterpret_cast<unsigned long long *>(bar);   // 8-byte aligned
-        const unsigned long long target = ++bar_epoch() * (unsigned long long)G;
-        // release: the block's writes (ordered before this thread by the
-        // __syncthreads above) are visible device-wide before the arrival
-        asm volatile("red.release.gpu.global.add.u64 [%0], 1;" ::"l"(cnt) : "memory");
-        const long long t0 = clock64(), lim = wait_limit_slot();
-        while (ld_acquire(cnt) < target) {
-            if (ld_volatile(err)) { ok = 0; break; }
-            if (clock64() - t0 > lim) { atomicExch(err, 1); ok = 0; break; }
-        }
-        // acquire: the load that saw the count completes before any later
-        // access of the block (the __syncthreads below orders the others)
-        asm volatile("fence.acq_rel.gpu;" ::: "memory");
-        if (ld_volatile(err)) ok = 0;
-        if (tm) { tm[T_BARRIER] += clock64() - tb; tm[T_BARRIERS]++; }
-    }
-    __syncthreads();
-    return ok;
-}
-
-template <typename T> __device__ __forceinline__ T ldcg(const T *p) { return __ldcg(p); }
-
-__device__ __forceinline__ double warp_sum(double v) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
-// maximum that keeps a NaN (fmax drops it): a non-finite residual must reach
-// the host as such, never as the other operand
-__device__ __forceinline__ double max_nan(double a, double b) { return a != a ? a : (b != b ? b : fmax(a, b)); }
-
-__device__ __forceinline__ float warp_sum(float v) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
 // block-reduce K (<= KMAX) per-thread values, result in red[off + l][0].
 // The warps reduce in the type of the values (FP32 in the mixed path: FP64
 // runs at a small fraction of the FP32 rate on this part), the NWARP warp
@@ -262,13 +179,6 @@ template <> struct Prec<float> {
     __device__ static const float *lr(const MgLevelDev &l) { return l.rw32; }
     __device__ static const float *ci(const MgDev &m) { return m.cinv32; }
 };
-
-// rows [r0, r1) of a level of size n split over G blocks
-__device__ __forceinline__ void own_rows(int n, int G, int bi, int &r0, int &r1) {
-    const int rpb = (n + G - 1) / G;
-    r0 = min(n, bi * rpb);
-    r1 = min(n, r0 + rpb);
-}
 
 // sum_k A[k][i] x[col]; CG: x read through L2 (written by other blocks).
 // All column/value loads of the row are issued together, then all gathers
@@ -495,6 +405,12 @@ __device__ __forceinline__ void smem_levels(const MgDev *__restrict__ mgp, VT *s
 // match and no CTA leaves while a peer may read its memory), or every CTA sees
 // the poison and none enters.  A cluster barrier at the end keeps each CTA's
 // memory alive until its peers are done with it.
+__device__ __forceinline__ unsigned long long ld_acquire(const unsigned long long *p) {
+    unsigned long long v;
+    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+
 constexpr unsigned long long CCNT_POISON = 1ull << 62;
 constexpr unsigned long long CCNT_MASK = (1ull << 40) - 1;
 
