@@ -24,8 +24,10 @@ UNITS = [
     ("phg_mesh.cpp", "host", []),
     ("phg_assemble.cpp", "host", []),
     ("phg_cache.cpp", "host", []),
+    ("phg_mgplan.cpp", "host", []),
     ("phg_kernels.cu", "cuda", ["-fmad=false"]),
     ("phg_gmres.cu", "cuda", []),
+    ("phg_mgs.cu", "cuda", []),
     ("phg_capi.cu", "cuda", []),
     ("phg_serve.cu", "cuda", []),
     ("phg_tune.cu", "cuda", []),

@@ -159,6 +159,18 @@ struct LevelData {
         if (!mg_ok) err = mg_err;
         return mg_ok ? &mg : nullptr;
     }
+    std::mutex plan_mu;              // the V-cycle's composed operators, for one omega
+    std::shared_ptr<const MgPlan> plan;
+    double plan_omega = 0.0;
+    std::shared_ptr<const MgPlan> mg_plan(const MgHierarchy &h, double omega) {
+        std::lock_guard<std::mutex> g(plan_mu);
+        if (plan && plan_omega == omega) return plan;
+        auto p = std::make_shared<MgPlan>();
+        if (!build_mg_plan(ops.lapl, h, omega, *p)) return nullptr;
+        plan = p;
+        plan_omega = omega;
+        return p;
+    }
 };
 
 struct phg_mesh_s {
@@ -481,6 +493,7 @@ struct MgLevelBufs {
 
 struct MgBufs {
     std::vector<std::unique_ptr<MgLevelBufs>> lev;
+    std::vector<std::unique_ptr<DBuf>> plan;   // the composed operators' tables
     DBuf cinv64, cinv32;
     DBuf desc;   // the MgDev descriptor in device memory
 };
@@ -662,12 +675,94 @@ std::vector<float> to_f32(const std::vector<T> &v) { return std::vector<float>(v
 int env_int(const char *name, int dflt) { const char *e = getenv(name); return e ? atoi(e) : dflt; }
 double env_dbl(const char *name, double dflt) { const char *e = getenv(name); return e ? atof(e) : dflt; }
 
+// the V-cycle's composed operators (phg_mgplan.cpp) in HBM, in the handle's precision
+int build_mgx_dev(phg_mesh_s *mh, const MgHierarchy &h, const MgDev &mg, SolveOpBufs &Lb, MgBufs &mb, int prec) {
+    std::shared_ptr<const MgPlan> pp = mh->d->mg_plan(h, mg.omega);
+    if (!pp) return PHG_OK;   // the solver then keeps the level-by-level V-cycle
+    const MgPlan &P = *pp;
+    MgxDev x;
+    mb.plan.clear();
+    auto fresh = [&]() -> DBuf & { mb.plan.emplace_back(new DBuf()); return *mb.plan.back(); };
+    auto values = [&](const std::vector<double> &v, const void **out) -> int {
+        DBuf &b = fresh();
+        if (prec == PHG_MIXED) CK(upload(b, to_f32(v)));
+        else CK(upload(b, v));
+        *out = b.p;
+        return PHG_OK;
+    };
+    // rows of W entries at a stride, padding (the row's first column, 0); the
+    // values of `on`, an operator whose pattern lies within c's (null: c itself)
+    auto rows_of = [&](const Csr &c, const Csr *on, int W, int stride, std::vector<int> *col, std::vector<double> &val) {
+        const int n = c.n;
+        if (col) col->assign((size_t)stride * n, 0);
+        val.assign((size_t)stride * n, 0.0);
+        bool fits = true;
+#pragma omp parallel for schedule(static) reduction(&& : fits)
+        for (int i = 0; i < n; ++i) {
+            const int q0 = c.ptr[i], len = c.ptr[i + 1] - q0;
+            if (len < 1 || len > W) { fits = false; continue; }
+            if (col)
+                for (int k = 0; k < stride; ++k) (*col)[(size_t)i * stride + k] = c.col[q0 + (k < len ? k : 0)];
+            const Csr &o = on ? *on : c;
+            for (int q = o.ptr[i]; q < o.ptr[i + 1]; ++q) {
+                int k = 0;
+                while (k < len && c.col[q0 + k] != o.col[q]) ++k;
+                if (k == len) { fits = false; break; }
+                val[(size_t)i * stride + k] = o.val[q];
+            }
+        }
+        return fits;
+    };
+    std::vector<int> col;
+    std::vector<double> val;
+    auto sparse = [&](const Csr &c, int W, int stride, const int **cols, const void **vals, bool *fits) -> int {
+        if (!(*fits = rows_of(c, nullptr, W, stride, &col, val))) return PHG_OK;
+        DBuf &b = fresh();
+        CK(upload(b, col));
+        *cols = b.as<int>();
+        return values(val, vals);
+    };
+    int r;
+    bool fits = true;   // other meshes keep the level-by-level V-cycle
+    for (int l = 0; l < mg.nlev; ++l) x.lev[l].n = mg.lev[l].n;
+    for (int l = 0; l + 1 < mg.nlev; ++l) {
+        MgxLevelDev &D = x.lev[l];
+        const MgPlan::Level &L = P.lev[l];
+        if ((r = sparse(L.T, MGX_WT, MGX_WT, &D.tc, &D.tv, &fits)) || !fits) return r;
+        if ((r = sparse(L.Q, MGX_WQ, MGX_WQ, &D.qc, &D.qv, &fits)) || !fits) return r;
+        if ((r = sparse(L.U, MGX_WU, MGX_WU, &D.uc, &D.uv, &fits)) || !fits) return r;
+    }
+    if (!rows_of(P.lev[0].T, &mh->ops.lapl, MGX_WT, MGX_WT, nullptr, val)) return PHG_OK;
+    if ((r = values(val, &x.a))) return r;
+    if ((r = sparse(P.AU, MGX_WF, MGX_SF, &x.fc, &x.fa, &fits)) || !fits) return r;
+    if (!rows_of(P.AU, &P.lev[0].U, MGX_WF, MGX_SF, nullptr, val)) return PHG_OK;
+    if ((r = values(val, &x.fu))) return r;
+    x.first_dense = P.first_dense;
+    auto dense = [&](const std::vector<double> &d, int m, const void **out) -> int {
+        const size_t rows = d.size() / m, st = mgx_stride(m);
+        std::vector<double> v(rows * st, 0.0);
+        for (size_t i = 0; i < rows; ++i) std::copy(&d[i * m], &d[i * m] + m, &v[i * st]);
+        return values(v, out);
+    };
+    for (int l = P.first_dense; l < mg.nlev; ++l)
+        if ((r = dense(P.B[l], mg.lev[l].n, &x.B[l]))) return r;
+    const int nd = mg.lev[P.first_dense].n;
+    // the wide dense product pays in FP32 only (FP64 multiply-adds are scarce)
+    if (prec == PHG_MIXED && !P.E.empty() && (r = dense(P.E, nd, &x.E))) return r;
+    if (!P.AB.empty() && (r = dense(P.AB, nd, &x.AB))) return r;
+    if (prec == PHG_MIXED && !P.AE.empty() && (r = dense(P.AE, nd, &x.AE))) return r;
+    x.nlev = mg.nlev;
+    Lb.op.mgx = x;
+    return PHG_OK;
+}
+
 // Geometric multigrid for the Laplacian of a generated icosahedral mesh:
 // levels down to the 42-point icosahedron refinement, Jacobi smoothing,
 // coarse levels of at most `red_max` points solved per block in shared memory.
 int build_mg_dev(phg_ops_s *o, phg_mesh_s *mh, SolveOpBufs &Lb, MgBufs &mb, int prec) {
     const Mesh &m = mh->m;
     Lb.op.mg = MgDev();
+    Lb.op.mgx = MgxDev();
     if (env_int("PHG_MG", 1) == 0 || m.level < 3) return PHG_OK;
     std::string err;
     const MgHierarchy *hp = mh->hierarchy(err);
@@ -806,6 +901,10 @@ int build_mg_dev(phg_ops_s *o, phg_mesh_s *mh, SolveOpBufs &Lb, MgBufs &mb, int 
                 mg.cl_elems = off;
             }
         }
+    }
+    if (mg.nu1 == 1) {
+        const int r = build_mgx_dev(mh, h, mg, Lb, mb, prec);
+        if (r) return r;
     }
     CK(mb.desc.ensure(sizeof(MgDev)));
     CK(cudaMemcpy(mb.desc.p, &mg, sizeof(MgDev), cudaMemcpyHostToDevice));
@@ -1362,6 +1461,15 @@ extern "C" int phg_ops_validate(phg_ops o, long long *bad_entries, void *stream)
             CK(check_range(D.rf, (long long)D.Wr * nc, -1, D.n, bad, s));
         }
     }
+    const MgxDev &mx = o->L.op.mgx;
+    for (int l = 0; l + 1 < mx.nlev; ++l) {
+        const MgxLevelDev &D = mx.lev[l];
+        const int nc = mx.lev[l + 1].n;
+        CK(check_range(D.tc, (long long)MGX_WT * D.n, 0, D.n, bad, s));
+        CK(check_range(D.qc, (long long)MGX_WQ * nc, 0, D.n, bad, s));
+        CK(check_range(D.uc, (long long)MGX_WU * D.n, 0, nc, bad, s));
+    }
+    if (mx.nlev) CK(check_range(mx.fc, (long long)MGX_SF * mx.lev[0].n, 0, mx.lev[1].n, bad, s));
     unsigned long long h = 0;
     CK(cudaMemcpyAsync(&h, bad, sizeof h, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
@@ -1412,7 +1520,7 @@ int time_best(cudaStream_t s, int reps, F fn, float *best) {
 }
 
 // the fastest launch shape of op's solves at nv right-hand sides b = A x*
-// (x* hashed), among rows per block 128..1024 and, for Chebyshev-solvable
+// (x* hashed), among rows per block 128..1024 (0: the built-in rule) and, for Chebyshev-solvable
 // operators in mixed precision with 8 or more right-hand sides, the lockstep
 // path; candidates that do not reach the tolerance are not chosen
 int tune_solve(phg_ops_s *o, const char *label, const DevSolveOp &op, int nv, cudaStream_t s, Report &rep) {
@@ -1425,7 +1533,7 @@ int tune_solve(phg_ops_s *o, const char *label, const DevSolveOp &op, int nv, cu
     CK(fill_hash(xs.as<double>(), (long long)len, 12345u + (unsigned)nv, s));
     CK(apply_op(op.A, DevCols(), xs.as<double>(), n, nullptr, nullptr, 0, nullptr, b.as<double>(), n, nv, s));
     std::vector<SolveShape> cand;
-    for (int rpb : {128, 256, 512, 1024}) { SolveShape c; c.rpb = rpb; c.path = 0; cand.push_back(c); }
+    for (int rpb : {0, 128, 256, 512, 1024}) { SolveShape c; c.rpb = rpb; c.path = 0; cand.push_back(c); }
     if ((fam == 1 || fam == 2) && pr == PREC_MIXED && nv >= 8) { SolveShape c; c.rpb = 0; c.path = 1; cand.push_back(c); }
     size_t need = 0;   // the largest workspace among the candidates' paths
     for (const SolveShape &c : cand) need = std::max(need, gmres_work_bytes(op, nv, o->restart, pr, &c));

@@ -66,6 +66,31 @@ struct MgDev {
     size_t cl_elems = 0;
 };
 
+// The V-cycle as composed operators (phg_mgplan.cpp), values in the handle's
+// precision.  Sparse rows have a fixed number of entries (the composed
+// stencils of a triangulation whose points have at most six neighbours), padded
+// with (the row's first column, 0), one row after the other: a block's rows
+// are one piece, a thread's row one short run, and the odd strides (4 lanes
+// share a row of Q) spread a warp's rows over all banks of shared memory.
+// Dense operators are row-major, rows padded with zeros to whole 16 bytes.
+constexpr int MGX_WT = 7, MGX_WU = 7, MGX_WQ = 20, MGX_WF = 10, MGX_SF = 11;   // entries; SF: row stride of F
+__host__ __device__ constexpr int mgx_stride(int n) { return (n + 3) & ~3; }
+struct MgxLevelDev {
+    int n = 0;
+    const int *qc = nullptr, *tc = nullptr, *uc = nullptr;      // Q: rows of level l + 1; T, U: rows of level l
+    const void *qv = nullptr, *tv = nullptr, *uv = nullptr;
+};
+struct MgxDev {
+    int nlev = 0;                    // 0 = not available
+    MgxLevelDev lev[MG_MAXLEV];
+    const void *a = nullptr;         // finest level: A on T's pattern
+    const int *fc = nullptr;         // finest level: U and A U on the pattern of A U
+    const void *fu = nullptr, *fa = nullptr;
+    int first_dense = 0;             // levels [first_dense, nlev) have B
+    const void *B[MG_MAXLEV] = {nullptr};
+    const void *E = nullptr, *AB = nullptr, *AE = nullptr;
+};
+
 // Operator of the Krylov solver: the exact A (FP64 residuals), Jacobi-scaled
 // copies A D^{-1} for the plain Jacobi path, and optionally a multigrid
 // V-cycle used as a flexible right preconditioner instead of Jacobi.
@@ -77,6 +102,7 @@ struct DevSolveOp {
     const float *a32 = nullptr;    // A in FP32 (multigrid path, mixed precision)
     MgDev mg;                      // host copy (sizes)
     const MgDev *mgd = nullptr;    // the same descriptor in device memory (read by the kernel)
+    MgxDev mgx;                    // the V-cycle's composed operators
     // Block preconditioner of a vertex-interleaved 4-field system (unknown
     // 4i+q, q = 0,1 "w" rows, q = 2,3 "u" rows whose diagonal blocks are -L):
     // z_w = D^-1 v_w, z_u = -Vcycle_L(v_u - M z_w); mgd is then the hierarchy

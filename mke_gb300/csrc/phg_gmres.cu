@@ -40,6 +40,7 @@
 
 #include "phg_group.cuh"
 #include "phg_kernels.cuh"
+#include "phg_mgs.cuh"
 
 namespace phg {
 
@@ -1261,7 +1262,9 @@ Layout layout(const DevSolveOp &op, int nv, int m, Precision prec) {
     L.mg = L.r + al(8 * (size_t)nv * n);
     const int groups = nv < GROUPS_CAP ? nv : GROUPS_CAP;
     const size_t ge = block_group_elems(op);
-    L.part = L.mg + (mg ? al(es * ge * (size_t)groups) : 0);
+    size_t gb = es * ge;   // per right-hand side in flight
+    if (mg && mgs_applicable(op)) gb = std::max(gb, mgs_scratch_bytes(op, prec));
+    L.part = L.mg + (mg ? al(gb * (size_t)groups) : 0);
     // groups * G <= co-resident blocks (< 4096)
     L.bar = L.part + al(8 * (size_t)4096 * 2 * (MAXM + 2));
     L.err = L.bar + al(8 * (size_t)GROUPS_CAP);
@@ -2588,6 +2591,23 @@ cudaError_t gmres_solve(const DevSolveOp &op, const double *B, double *X, int nv
         e0 = cheb_lockstep(op, B, X, nv, ld, tol, ev ? atof(ev) : INNER_RTOL, (char *)work,
                            layout(op, nv, m, prec), stats_dev, s);
         if (e0 != cudaErrorNotSupported) return e0;
+    }
+    if (!cheb && op.mgd && mgs_applicable(op)) {
+        const Layout L = layout(op, nv, m, prec);
+        char *w = (char *)work;
+        cudaError_t e0;
+        if ((e0 = cudaMemsetAsync(w + L.bar, 0, L.total - L.bar, s)) != cudaSuccess) return e0;
+        if ((e0 = cudaMemsetAsync(stats_dev, 0, sizeof(GmresStats), s)) != cudaSuccess) return e0;
+        MgsArgs a;
+        a.B = B; a.X = X; a.nv = nv; a.ld = ld; a.m = m; a.max_iter = max_iter; a.tol = tol;
+        const char *ev = getenv("PHG_INNER_RTOL");
+        a.inner_rtol = ev ? atof(ev) : INNER_RTOL;
+        a.prec = prec; a.rpb = sh.rpb; a.sms = sm_count(); a.max_sms = max_sms;
+        a.wait_limit = wait_limit > 0 ? wait_limit : SPIN_LIMIT;
+        a.V = w + L.v; a.Z = w + L.z; a.Wv = w + L.w; a.R = (double *)(w + L.r);
+        a.scratch = w + L.mg; a.part = (double *)(w + L.part);
+        a.bar = (unsigned *)(w + L.bar); a.err = (int *)(w + L.err); a.stats = stats_dev;
+        return mgs_solve(op, a, s);
     }
     // cluster tail of the V-cycle: the levels [ncl, nred) in the group's first
     // cluster (needs a group of at least one whole cluster, see below)

@@ -100,6 +100,23 @@ struct MgHierarchy {
     std::vector<double> coarse_inv;  // dense inverse of the coarsest A (row-major)
 };
 bool build_mg(const Mesh &fine, int coarsest_level, MgHierarchy &h, std::string &err);
+
+// The V-cycle (one damped-Jacobi sweep down and one up, dense coarsest solve)
+// as composed operators (phg_mgplan.cpp): per level l < nlev - 1 the sparse
+// Q (level l to l + 1), T and U, from level first_dense on the dense V-cycle
+// matrices B (row-major); AU = A U of the finest level; E = U B across levels
+// first_dense - 1 and first_dense where that is not too large; A B and A E
+// where they start at the finest level.
+constexpr int MG_DENSE_ROWS = 700, MG_WIDE_ROWS = 2600;
+struct MgPlan {
+    struct Level { Csr Q, T, U; };
+    std::vector<Level> lev;
+    Csr AU;
+    int first_dense = 0;
+    std::vector<std::vector<double>> B;
+    std::vector<double> E, AB, AE;
+};
+bool build_mg_plan(const Csr &fine, const MgHierarchy &h, double omega, MgPlan &p);
 // BarVortex forward matrix c1 * mass + c2 * slaplace (examples/barvortex_impl.h:57-78)
 void assemble_barvortex(const Mesh &m, double c1, double c2, Csr &A, Csr &Abnd);
 // Baroclin 4rs x 4rs block matrix (examples/baroclin.cpp:119-180) and the
