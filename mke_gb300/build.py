@@ -28,6 +28,7 @@ UNITS = [
     ("phg_kernels.cu", "cuda", ["-fmad=false"]),
     ("phg_gmres.cu", "cuda", []),
     ("phg_mgs.cu", "cuda", []),
+    ("phg_chs.cu", "cuda", []),
     ("phg_capi.cu", "cuda", []),
     ("phg_serve.cu", "cuda", []),
     ("phg_tune.cu", "cuda", []),

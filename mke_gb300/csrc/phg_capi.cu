@@ -482,6 +482,7 @@ void to_ell(const Csr &c, int W, std::vector<int> *col, std::vector<double> &val
 
 struct SolveOpBufs {
     DBuf val, as64, as32, a32, dinv, dinv32;
+    DBuf c7, v7;   // D^-1 A by rows of seven (Chebyshev-solvable operators)
     DBuf pk;   // FP32 row records for the interleaved apply: 8 (column, value) pairs per row
     DevSolveOp op;
 };
@@ -647,6 +648,36 @@ int build_solve_op(phg_ops_s *o, const Csr &c, SolveOpBufs &b, bool try_cheb = f
     if (try_cheb && o->W <= 8 && env_int("PHG_CHEB", 1)) {
         double lo = 0.0, hi = 0.0;
         if (cheb_interval(c, dinv, lo, hi)) { b.op.cheb_lmin = lo; b.op.cheb_lmax = hi; }
+    }
+    b.op.c7 = nullptr;
+    b.op.v7 = nullptr;
+    if (b.op.cheb_lmax > 0.0) {
+        // D^-1 A by rows, the diagonal first; only for symmetric patterns
+        // (phg_chs.cu says why) of at most seven entries a row
+        std::vector<int> c7((size_t)7 * n);
+        std::vector<double> v7((size_t)7 * n, 0.0);
+        bool fits = true;
+#pragma omp parallel for schedule(static) reduction(&& : fits)
+        for (int i = 0; i < n; ++i) {
+            if (c.ptr[i + 1] - c.ptr[i] > 7) { fits = false; continue; }
+            int k = 1;
+            for (int q = 0; q < 7; ++q) c7[(size_t)7 * i + q] = i;
+            for (int q = c.ptr[i]; q < c.ptr[i + 1]; ++q) {
+                const int j = c.col[q];
+                const int at = j == i ? 0 : k++;
+                if (at > 6) { fits = false; break; }
+                c7[(size_t)7 * i + at] = j;
+                v7[(size_t)7 * i + at] = dinv[i] * c.val[q];
+                fits = fits && std::binary_search(&c.col[c.ptr[j]], &c.col[c.ptr[j]] + (c.ptr[j + 1] - c.ptr[j]), i);
+            }
+        }
+        if (fits) {
+            CK(upload(b.c7, c7));
+            if (o->prec == PHG_MIXED) CK(upload(b.v7, std::vector<float>(v7.begin(), v7.end())));
+            else CK(upload(b.v7, v7));
+            b.op.c7 = b.c7.as<int>();
+            b.op.v7 = b.v7.p;
+        }
     }
     return PHG_OK;
 }
@@ -1461,6 +1492,8 @@ extern "C" int phg_ops_validate(phg_ops o, long long *bad_entries, void *stream)
             CK(check_range(D.rf, (long long)D.Wr * nc, -1, D.n, bad, s));
         }
     }
+    for (const DevSolveOp *op : {&o->ML.op, &o->MJ.op})
+        if (op->c7) CK(check_range(op->c7, 7LL * op->A.n, 0, op->A.n, bad, s));
     const MgxDev &mx = o->L.op.mgx;
     for (int l = 0; l + 1 < mx.nlev; ++l) {
         const MgxLevelDev &D = mx.lev[l];

@@ -116,6 +116,10 @@ struct DevSolveOp {
     // set, the solver runs Chebyshev iterations inside the FP64 refinement
     // loop instead of GMRES -- no inner products, one group barrier per step.
     double cheb_lmin = 0.0, cheb_lmax = 0.0;
+    // D^-1 A by rows of seven entries, the diagonal first, padded with (i, 0),
+    // in the handle's precision; null unless the pattern is symmetric
+    const int *c7 = nullptr;
+    const void *v7 = nullptr;
     // FP32 row records of A (8 (column, value) pairs per row, padding (i, 0)):
     // one sequential matrix stream for the lockstep kernels; null if absent
     const uint4 *pk32 = nullptr;
@@ -153,7 +157,7 @@ struct GmresStats {
 // (no block gets fewer rows; 0 = 256).  path, for Chebyshev-solvable
 // operators in mixed precision: 1 = lockstep launches over an interleaved
 // FP32 multi-vector (8 or more right-hand sides), 0 = per-member persistent
-// kernels, -1 = the built-in rule (lockstep from 32 right-hand sides).
+// kernels, -1 = the built-in rule (by rows x right-hand sides, choose_path).
 struct SolveShape {
     int rpb = 0;
     int path = -1;

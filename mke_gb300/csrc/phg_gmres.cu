@@ -40,6 +40,7 @@
 
 #include "phg_group.cuh"
 #include "phg_kernels.cuh"
+#include "phg_chs.cuh"
 #include "phg_mgs.cuh"
 
 namespace phg {
@@ -51,15 +52,14 @@ namespace {
 constexpr int BLOCK = 256;
 constexpr int NWARP = BLOCK / 32;
 constexpr double INNER_RTOL = 1e-5;  // FP32 cycle: reduce the residual 1e5x, then refine
-constexpr int CHEB_KMAX = 64;    // most Chebyshev steps per refinement cycle
-constexpr int LS_MIN_RHS = 32;   // right-hand sides from which the lockstep path runs
-constexpr int LS_MIN_TUNED = 8;  // the fewest for which the autotuner may choose it
-// the multigrid Laplacian runs in lockstep by default from this many
-// right-hand sides on meshes of at least LSG_DEFAULT_ROWS rows (measured,
-// graph-replayed ensemble steps: L5 x 256 -15 %, L6 x 32 -14 %, L7 x 16 -5 %,
-// but L4 x 64 +9 %); elsewhere only when the autotuner chose it
-constexpr int LSG_DEFAULT_RHS = 16;
-constexpr int LSG_DEFAULT_ROWS = 10000;
+constexpr int LS_MIN_TUNED = 8;  // the fewest right-hand sides for which the autotuner may choose a lockstep path
+// Lockstep launches over all right-hand sides (one short kernel per phase,
+// streaming) or the persistent kernels (phg_chs.cu, phg_mgs.cu): the latter
+// keep a few right-hand sides' vectors on chip and hand them from block to
+// block, the former win once the vectors outgrow that -- by rows x right-hand
+// sides, from about these products on (measured; see choose_path)
+constexpr long long LS_MIN_WORK = 8000000;    // Chebyshev solves
+constexpr long long LSG_MIN_WORK = 2000000;   // multigrid Laplacians
 
 // One operator's share of a multi-operator launch (meshes of several levels
 // in one persistent launch): right-hand sides [v0, next v0) use this
@@ -1232,6 +1232,8 @@ size_t block_group_elems(const DevSolveOp &op) {
     return 2 * op.mg.group_elems + 4 * (size_t)(op.A.n / 4);
 }
 
+int sm_count();
+
 // whether gmres_solve runs op's solves as Chebyshev iterations (the same test)
 bool uses_cheb(const DevSolveOp &op, int m) {
     return op.cheb_lmax > 0.0 && op.cheb_lmin > 0.0 && op.cheb_lmin < op.cheb_lmax && m >= 3 && !op.mgd &&
@@ -1249,7 +1251,7 @@ Layout layout(const DevSolveOp &op, int nv, int m, Precision prec) {
     // path needs three interleaved FP32 vectors and the norm partials instead
     size_t vregion = es * (size_t)nv * (m + 1) * n;
     if (uses_cheb(op, m)) {
-        vregion = es * (size_t)nv * 4 * n;
+        vregion = op.c7 ? chs_work_bytes(op, nv, prec, sm_count()) : es * (size_t)nv * 4 * n;
         if (prec == PREC_MIXED) {
             const size_t nvp = (size_t)(nv + 31) / 32 * 32, nbx = ((size_t)n + 255) / 256;
             vregion = std::max(vregion, 3 * al(4 * (size_t)n * nvp) + 16 * (size_t)nv * nbx);
@@ -1258,7 +1260,7 @@ Layout layout(const DevSolveOp &op, int nv, int m, Precision prec) {
     L.v = 0;
     L.z = L.v + al(vregion);
     L.w = L.z + (mg ? al(es * (size_t)nv * m * n) : 0);
-    L.r = L.w + al(es * (size_t)nv * n);
+    L.r = L.w + (uses_cheb(op, m) ? 0 : al(es * (size_t)nv * n));
     L.mg = L.r + al(8 * (size_t)nv * n);
     const int groups = nv < GROUPS_CAP ? nv : GROUPS_CAP;
     const size_t ge = block_group_elems(op);
@@ -1554,8 +1556,6 @@ __global__ void __launch_bounds__(256) k_ls_update(double *X, int ld, int n, int
     }
 }
 
-int sm_count();
-
 // Blocks of 256 threads resident at once for `kernel`: the grid of a
 // grid-stride lockstep launch.  The launches of cycles after convergence only
 // read the stop flag, and a full-size grid (one block per 256 work items)
@@ -1633,21 +1633,10 @@ cudaError_t cheb_lockstep(const DevSolveOp &op, const double *B, double *X, int 
     double *R = (double *)(w + L.r);
     double *nrm = (double *)(w + L.part), *beta = nrm + 2 * nvp, *sc = beta + nvp;
     int *done = (int *)(sc + nvp), *kcp = done + 1;   // stop flag; the cycle's steps
-    // coefficients (as the per-member Chebyshev kernel)
-    const double lo = op.cheb_lmin, hi = op.cheb_lmax;
-    const double kappa = hi / lo, sq = sqrt(kappa), sigma = (sq - 1.0) / (sq + 1.0);
-    int K = (int)ceil(log(2.0 * kappa / inner_rtol) / log(1.0 / sigma)) + 1;
-    K = K < 2 ? 2 : (K > CHEB_KMAX ? CHEB_KMAX : K);
-    const double lg = log(2.0 * kappa), ls = log(1.0 / sigma);
-    const double theta = 0.5 * (hi + lo), delta = 0.5 * (hi - lo), s1 = theta / delta;
-    double ca[CHEB_KMAX], cb[CHEB_KMAX], rho_prev = 1.0 / s1;
-    ca[0] = cb[0] = 0.0;
-    for (int k = 1; k < K; ++k) {
-        const double rho = 1.0 / (2.0 * s1 - rho_prev);
-        ca[k] = rho * rho_prev;
-        cb[k] = 2.0 * rho / delta;
-        rho_prev = rho;
-    }
+    ChebPlan pl;
+    cheb_plan(op, inner_rtol, pl);
+    const int K = pl.K;
+    const double lg = pl.lg, ls = pl.ls, *ca = pl.ca, *cb = pl.cb;
     // algorithmic bytes of one cycle: FP64 residual, init, K - 1 steps, update
     const double rowsb = (double)n;
     const double cyc = rowsb * nv * (8.0 * 3) + rowsb * W * 12.0 +
@@ -1669,7 +1658,7 @@ cudaError_t cheb_lockstep(const DevSolveOp &op, const double *B, double *X, int 
         k_ls_nrm<<<(nv + NWARP - 1) / NWARP, 256, 0, s>>>(rpart, bpart, nbx, nrm, nv, done);
         k_ls_scale<<<1, 256, 0, s>>>(nrm, nv, nvp, tol, beta, sc, done, st, c, K, c ? cyc : 0.0, lg, ls, kcp);
         if (c == LS_MAXC) break;
-        k_ls_init<<<capped(ntile, cap_init), 256, 0, s>>>(R, n, nv, nvp, sc, op.dinv32, (float)(1.0 / theta), rv, e0,
+        k_ls_init<<<capped(ntile, cap_init), 256, 0, s>>>(R, n, nv, nvp, sc, op.dinv32, (float)pl.c0, rv, e0,
                                                           e1, done);
         float *ec = e1, *ep = e0;
         switch (W) {
@@ -2510,6 +2499,26 @@ cudaError_t lsg_solve(const DevSolveOp &op, const double *B, double *X, int nv, 
 
 }  // namespace
 
+void cheb_plan(const DevSolveOp &op, double eps, ChebPlan &p) {
+    // steps for an error reduction eps (residual: one more factor kappa)
+    const double lo = op.cheb_lmin, hi = op.cheb_lmax;
+    const double kappa = hi / lo, sq = sqrt(kappa), sigma = (sq - 1.0) / (sq + 1.0);
+    const int K = (int)ceil(log(2.0 * kappa / eps) / log(1.0 / sigma)) + 1;
+    p.K = K < 2 ? 2 : (K > CHEB_KMAX ? CHEB_KMAX : K);
+    p.lg = log(2.0 * kappa);
+    p.ls = log(1.0 / sigma);
+    const double theta = 0.5 * (hi + lo), delta = 0.5 * (hi - lo), s1 = theta / delta;
+    p.c0 = 1.0 / theta;
+    double rho_prev = 1.0 / s1;
+    for (int k = 0; k < CHEB_KMAX; ++k) p.ca[k] = p.cb[k] = 0.0;
+    for (int k = 1; k < p.K; ++k) {
+        const double rho = 1.0 / (2.0 * s1 - rho_prev);
+        p.ca[k] = rho * rho_prev;
+        p.cb[k] = 2.0 * rho / delta;
+        rho_prev = rho;
+    }
+}
+
 // The kernels may use all the opt-in shared memory; set once per kernel, so
 // that threads launching with different sizes never race on the attribute.
 static cudaError_t allow_smem(Precision prec, bool multi = false) {
@@ -2543,12 +2552,15 @@ SolvePath choose_path(const DevSolveOp &op, int nv, int m, Precision prec, bool 
     if (getenv("PHG_CHEB_LOCKSTEP") && !env_int("PHG_CHEB_LOCKSTEP", 1)) sh.path = 0;
     if (sh_out) *sh_out = sh;
     if (no_alloc) return SolvePath::Persistent;
+    // Level 5, mixed: 100 Laplace solves 2.7 ms persistent, 3.6 ms lockstep;
+    // 256 of them 7.4 and 5.5 ms.  Level 6: 37 of them 4.2 and 6.0 ms, 64 of
+    // them 8.4 and 6.1 ms.
+    const long long work = (long long)op.A.n * nv;
     if (uses_cheb(op, m)) {
-        const bool ls = sh.path == 1 ? nv >= LS_MIN_TUNED : (sh.path == 0 ? false : nv >= LS_MIN_RHS);
+        const bool ls = sh.path == 1 ? nv >= LS_MIN_TUNED : (sh.path == 0 ? false : work >= LS_MIN_WORK && nv >= 32);
         return prec == PREC_MIXED && ls ? SolvePath::ChebLockstep : SolvePath::Persistent;
     }
-    if (lsg_applicable(op, nv, prec, m) &&
-        (sh.path == 1 || (sh.path == -1 && nv >= LSG_DEFAULT_RHS && op.A.n >= LSG_DEFAULT_ROWS)))
+    if (lsg_applicable(op, nv, prec, m) && (sh.path == 1 || (sh.path == -1 && work >= LSG_MIN_WORK)))
         return SolvePath::MgLockstep;
     return SolvePath::Persistent;
 }
@@ -2591,6 +2603,23 @@ cudaError_t gmres_solve(const DevSolveOp &op, const double *B, double *X, int nv
         e0 = cheb_lockstep(op, B, X, nv, ld, tol, ev ? atof(ev) : INNER_RTOL, (char *)work,
                            layout(op, nv, m, prec), stats_dev, s);
         if (e0 != cudaErrorNotSupported) return e0;
+    }
+    if (cheb && op.c7) {
+        const Layout L = layout(op, nv, m, prec);
+        char *w = (char *)work;
+        cudaError_t e0;
+        if ((e0 = cudaMemsetAsync(w + L.bar, 0, L.total - L.bar, s)) != cudaSuccess) return e0;
+        if ((e0 = cudaMemsetAsync(stats_dev, 0, sizeof(GmresStats), s)) != cudaSuccess) return e0;
+        const char *ev = getenv("PHG_INNER_RTOL");
+        ChebPlan pl;
+        cheb_plan(op, prec == PREC_MIXED ? (ev ? atof(ev) : INNER_RTOL) : fmax(0.25 * tol, 1e-15), pl);
+        ChsArgs a;
+        a.B = B; a.X = X; a.nv = nv; a.ld = ld; a.max_iter = max_iter; a.tol = tol;
+        a.prec = prec; a.plan = &pl; a.rpb = sh.rpb; a.sms = sm_count(); a.max_sms = max_sms;
+        a.wait_limit = wait_limit > 0 ? wait_limit : SPIN_LIMIT;
+        a.work = w + L.v; a.R = (double *)(w + L.r); a.part = (double *)(w + L.part);
+        a.bar = (unsigned *)(w + L.bar); a.err = (int *)(w + L.err); a.stats = stats_dev;
+        return chs_solve(op, a, s);
     }
     if (!cheb && op.mgd && mgs_applicable(op)) {
         const Layout L = layout(op, nv, m, prec);
@@ -2670,25 +2699,11 @@ cudaError_t gmres_solve(const DevSolveOp &op, const double *B, double *X, int nv
     p.cheb_k = 0;
     p.cheb_lg = p.cheb_ls = 0.0;
     if (cheb) {
-        // steps for an error reduction eps (residual: one more factor kappa)
-        const double lo = op.cheb_lmin, hi = op.cheb_lmax;
-        const double kappa = hi / lo, sq = sqrt(kappa), sigma = (sq - 1.0) / (sq + 1.0);
-        const double eps = prec == PREC_MIXED ? p.inner_rtol : fmax(0.25 * tol, 1e-15);
-        int K = (int)ceil(log(2.0 * kappa / eps) / log(1.0 / sigma)) + 1;
-        K = K < 2 ? 2 : (K > CHEB_KMAX ? CHEB_KMAX : K);
-        const double theta = 0.5 * (hi + lo), delta = 0.5 * (hi - lo), s1 = theta / delta;
-        p.cheb_k = K;
-        p.cheb_lg = log(2.0 * kappa);
-        p.cheb_ls = log(1.0 / sigma);
-        p.cheb_c0 = 1.0 / theta;
-        double rho_prev = 1.0 / s1;
-        p.cheb_ca[0] = p.cheb_cb[0] = 0.0;
-        for (int k = 1; k < K; ++k) {
-            const double rho = 1.0 / (2.0 * s1 - rho_prev);
-            p.cheb_ca[k] = rho * rho_prev;
-            p.cheb_cb[k] = 2.0 * rho / delta;
-            rho_prev = rho;
-        }
+        ChebPlan pl;
+        cheb_plan(op, prec == PREC_MIXED ? p.inner_rtol : fmax(0.25 * tol, 1e-15), pl);
+        p.cheb_k = pl.K; p.cheb_c0 = pl.c0; p.cheb_lg = pl.lg; p.cheb_ls = pl.ls;
+        memcpy(p.cheb_ca, pl.ca, sizeof pl.ca);
+        memcpy(p.cheb_cb, pl.cb, sizeof pl.cb);
     }
     p.part = (double *)(w + L.part);
     p.bar = (unsigned *)(w + L.bar); p.err = (int *)(w + L.err); p.stats = stats_dev;

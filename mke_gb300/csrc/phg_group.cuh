@@ -92,6 +92,29 @@ __device__ __forceinline__ float warp_sum(float v) {
     return v;
 }
 
+// the warp's sums of eight values per lane with 9 additions instead of 40:
+// halves exchange four, two and one of them, then two plain steps; lane l
+// returns the sum of value (l >> 2) & 7 (bit-reversed pairs, see the caller)
+template <typename T>
+__device__ __forceinline__ T fold8(const T (&t)[8], int lane) {
+    T a[4], b[2];
+    const bool h16 = lane & 16, h8 = lane & 8, h4 = lane & 4;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) a[k] = (h16 ? t[k + 4] : t[k]) + __shfl_xor_sync(0xffffffffu, h16 ? t[k] : t[k + 4], 16);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) b[k] = (h8 ? a[k + 2] : a[k]) + __shfl_xor_sync(0xffffffffu, h8 ? a[k] : a[k + 2], 8);
+    T c = (h4 ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, h4 ? b[0] : b[1], 4);
+    c += __shfl_xor_sync(0xffffffffu, c, 2);
+    c += __shfl_xor_sync(0xffffffffu, c, 1);
+    return c;   // value 4 (lane >> 4 & 1) + 2 (lane >> 3 & 1) + (lane >> 2 & 1)
+}
+
+// sum over the first `na` lanes (a power-of-two tree no larger than needed), in every lane
+__device__ __forceinline__ double lanes_sum(double v, int na) {
+    for (int o = 1; o < na; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return __shfl_sync(0xffffffffu, v, 0);
+}
+
 // maximum that keeps a NaN (fmax drops it): a non-finite residual must reach
 // the host as such, never as the other operand
 __device__ __forceinline__ double max_nan(double a, double b) { return a != a ? a : (b != b ? b : fmax(a, b)); }

@@ -96,61 +96,19 @@ template <typename VT> struct Rows {
     int base;
 };
 
-template <typename VT, bool ONE> struct Store;
-template <typename VT> struct Store<VT, true> {
-    using E = VT;
-    __device__ static void put(E *p, VT v, unsigned) { *p = v; }
-    template <int N>
-    __device__ static void get(VT (&x)[N], const E *p, const int (&c)[N], unsigned, const Waits &) {
-#pragma unroll
-        for (int q = 0; q < N; ++q) x[q] = p[c[q]];
-    }
-};
-template <typename VT> struct Store<VT, false> {
-    using E = Cell<VT>;
-    __device__ static void put(E *p, VT v, unsigned stamp) { st_cell(p, v, stamp); }
-    template <int N>
-    __device__ static void get(VT (&x)[N], const E *p, const int (&c)[N], unsigned stamp, const Waits &w) {
-        wait_cells<VT, N>(x, p, c, stamp, w);
-    }
-};
-
 // sum over N entries k = k0, k0 + KS, ... of row i: v[k] x[c[k]]
 template <typename VT, bool ONE, int N, int KS = 1>
-__device__ __forceinline__ VT row_sum(const int *col, const VT *v, const typename Store<VT, ONE>::E *p, unsigned stamp,
+__device__ __forceinline__ VT row_sum(const int *col, const VT *v, const typename CellStore<VT, ONE>::E *p, unsigned stamp,
                                       const Waits &w) {
     int c[N];
     VT x[N];
 #pragma unroll
     for (int q = 0; q < N; ++q) c[q] = col[KS * q];
-    Store<VT, ONE>::get(x, p, c, stamp, w);
+    CellStore<VT, ONE>::get(x, p, c, stamp, w);
     VT s = 0;
 #pragma unroll
     for (int q = 0; q < N; ++q) s += v[KS * q] * x[q];
     return s;
-}
-
-// the warp's sums of eight values per lane with 9 additions instead of 40:
-// halves exchange four, two and one of them, then two plain steps; lane l
-// returns the sum of value (l >> 2) & 7 (bit-reversed pairs, see the caller)
-template <typename T>
-__device__ __forceinline__ T fold8(const T (&t)[8], int lane) {
-    T a[4], b[2];
-    const bool h16 = lane & 16, h8 = lane & 8, h4 = lane & 4;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) a[k] = (h16 ? t[k + 4] : t[k]) + __shfl_xor_sync(0xffffffffu, h16 ? t[k] : t[k + 4], 16);
-#pragma unroll
-    for (int k = 0; k < 2; ++k) b[k] = (h8 ? a[k + 2] : a[k]) + __shfl_xor_sync(0xffffffffu, h8 ? a[k] : a[k + 2], 8);
-    T c = (h4 ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, h4 ? b[0] : b[1], 4);
-    c += __shfl_xor_sync(0xffffffffu, c, 2);
-    c += __shfl_xor_sync(0xffffffffu, c, 1);
-    return c;   // value 4 (lane >> 4 & 1) + 2 (lane >> 3 & 1) + (lane >> 2 & 1)
-}
-
-// sum over the first `na` lanes (a power-of-two tree no larger than needed), in every lane
-__device__ __forceinline__ double lanes_sum(double v, int na) {
-    for (int o = 1; o < na; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return __shfl_sync(0xffffffffu, v, 0);
 }
 
 // a dense row (16-byte aligned, length a multiple of four) times b, in every lane
@@ -200,7 +158,7 @@ __device__ __noinline__ VT root_sum(const Cell<VT> *part, int G, unsigned stamp,
 
 template <typename VT, bool ONE>
 __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(const __grid_constant__ MgsParams p) {
-    using ST = Store<VT, ONE>;
+    using ST = CellStore<VT, ONE>;
     using E = typename ST::E;
     extern __shared__ __align__(16) char smem[];
     double *H = (double *)smem;              // (m + 1) x m, the R factor
@@ -799,9 +757,12 @@ cudaError_t mgs_solve(const DevSolveOp &op, const MgsArgs &q, cudaStream_t s) {
     const size_t es = mixed ? 4 : 8;
     const int sms = (q.max_sms > 0 && q.max_sms < q.sms) ? q.max_sms : q.sms;
     // One block per SM with all its shared memory, its warps split over the
-    // rows; more right-hand sides than SMs: two smaller blocks per SM, one
-    // right-hand side each.
-    const bool many = q.nv > sms;
+    // rows; two smaller blocks per SM where that spreads the right-hand sides
+    // better: more of them than SMs, or more than half as many but few enough
+    // for three blocks each (level 5, 100 FP64 right-hand sides: 6.4 ms with one
+    // block each on 100 of 152 SMs, 4.3 ms with three half-size blocks; level 4,
+    // 152 mixed ones: 0.92 ms with one block, 1.20 ms with two halves).
+    const bool many = q.nv > sms || (2 * q.nv > sms && 2 * sms / q.nv >= 3);
     int workers = many ? 256 : (mixed ? 768 : 512);
     const int cap = many ? 2 * sms : sms;
     const int groups = std::min(q.nv, cap);

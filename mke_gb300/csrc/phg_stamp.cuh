@@ -94,6 +94,34 @@ __device__ __forceinline__ void wait_cells(VT (&x)[N], const Cell<VT> *p, const 
     }
 }
 
+// A vector whose elements are handed from block to block (stamped cells), or,
+// when one block owns every row (ONE), plain values ordered by __syncthreads.
+template <typename VT, bool ONE> struct CellStore;
+template <typename VT> struct CellStore<VT, true> {
+    using E = VT;
+    __device__ static void put(E *p, VT v, unsigned) { *p = v; }
+    template <int N>
+    __device__ static void get(VT (&x)[N], const E *p, const int (&c)[N], unsigned, const Waits &) {
+#pragma unroll
+        for (int q = 0; q < N; ++q) x[q] = p[c[q]];
+    }
+    __device__ static VT own(const E *p) { return *p; }
+};
+template <typename VT> struct CellStore<VT, false> {
+    using E = Cell<VT>;
+    __device__ static void put(E *p, VT v, unsigned stamp) { st_cell(p, v, stamp); }
+    template <int N>
+    __device__ static void get(VT (&x)[N], const E *p, const int (&c)[N], unsigned stamp, const Waits &w) {
+        wait_cells<VT, N>(x, p, c, stamp, w);
+    }
+    __device__ static VT own(const E *p) {   // written by this block before its last __syncthreads
+        VT v;
+        unsigned e;
+        ld_cell(p, v, e);
+        return v;
+    }
+};
+
 }  // namespace
 
 }  // namespace phg

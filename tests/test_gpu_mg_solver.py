@@ -77,3 +77,25 @@ def test_rows_per_block(monkeypatch):
     for rows in ("64", "1000", "20000"):
         monkeypatch.setenv("PHG_ROWS_PER_BLOCK", rows)
         check(m, ops, F, bnd, inner, want)
+
+
+@pytest.mark.parametrize("precision", [phelm.PHG_FP64, phelm.PHG_MIXED])
+@pytest.mark.parametrize("level", [2, 3, 4, 5])
+@pytest.mark.parametrize("members,sms", [(1, 0), (2, 1), (3, 0), (3, 7), (5, 150), (9, 0), (160, 0)])
+def test_mass_solves(level, precision, members, sms):
+    """The persistent Chebyshev solver (phg_chs.cu) through the barotropic
+    step: members (so 1 to 1,280 right-hand sides a solve, chunks of 1, 2, 4
+    and 8) over one, a few and all SMs, against the members' own single steps;
+    both solve to 1e-12, and 1e-9 is the bound of every step comparison."""
+    if members == 160 and level > 3:
+        pytest.skip("covered by the smaller meshes")
+    m = phelm.Mesh.sphere(level)
+    lat, lon = m.latlon()
+    u = serve.barvortex_inputs(lat, lon, members, seed=9)
+    ops = phelm.Operators(m, precision, tol=1e-12)
+    bv = phelm.BarVortex(ops, coriolis=np.sin(lat))
+    single = {k: bv.calc(u[k]) for k in {0, members // 2, members - 1}}
+    ops.set_sms(sms)
+    got = bv.calc_batch(u)
+    for k, want in single.items():
+        assert np.linalg.norm(got[k] - want) <= 1e-9 * np.linalg.norm(want), k
