@@ -706,6 +706,31 @@ std::vector<float> to_f32(const std::vector<T> &v) { return std::vector<float>(v
 int env_int(const char *name, int dflt) { const char *e = getenv(name); return e ? atoi(e) : dflt; }
 double env_dbl(const char *name, double dflt) { const char *e = getenv(name); return e ? atof(e) : dflt; }
 
+// rows of W entries at a stride, padding (the row's first column, 0); the
+// values of `on`, an operator whose pattern lies within c's (null: c itself).
+// False when a row has none or more than W entries, or does not fit.
+bool rows_of(const Csr &c, const Csr *on, int W, int stride, std::vector<int> *col, std::vector<double> &val) {
+    const int n = c.n;
+    if (col) col->assign((size_t)stride * n, 0);
+    val.assign((size_t)stride * n, 0.0);
+    bool fits = true;
+#pragma omp parallel for schedule(static) reduction(&& : fits)
+    for (int i = 0; i < n; ++i) {
+        const int q0 = c.ptr[i], len = c.ptr[i + 1] - q0;
+        if (len < 1 || len > W) { fits = false; continue; }
+        if (col)
+            for (int k = 0; k < stride; ++k) (*col)[(size_t)i * stride + k] = c.col[q0 + (k < len ? k : 0)];
+        const Csr &o = on ? *on : c;
+        for (int q = o.ptr[i]; q < o.ptr[i + 1]; ++q) {
+            int k = 0;
+            while (k < len && c.col[q0 + k] != o.col[q]) ++k;
+            if (k == len) { fits = false; break; }
+            val[(size_t)i * stride + k] = o.val[q];
+        }
+    }
+    return fits;
+}
+
 // the V-cycle's composed operators (phg_mgplan.cpp) in HBM, in the handle's precision
 int build_mgx_dev(phg_mesh_s *mh, const MgHierarchy &h, const MgDev &mg, SolveOpBufs &Lb, MgBufs &mb, int prec) {
     std::shared_ptr<const MgPlan> pp = mh->d->mg_plan(h, mg.omega);
@@ -720,29 +745,6 @@ int build_mgx_dev(phg_mesh_s *mh, const MgHierarchy &h, const MgDev &mg, SolveOp
         else CK(upload(b, v));
         *out = b.p;
         return PHG_OK;
-    };
-    // rows of W entries at a stride, padding (the row's first column, 0); the
-    // values of `on`, an operator whose pattern lies within c's (null: c itself)
-    auto rows_of = [&](const Csr &c, const Csr *on, int W, int stride, std::vector<int> *col, std::vector<double> &val) {
-        const int n = c.n;
-        if (col) col->assign((size_t)stride * n, 0);
-        val.assign((size_t)stride * n, 0.0);
-        bool fits = true;
-#pragma omp parallel for schedule(static) reduction(&& : fits)
-        for (int i = 0; i < n; ++i) {
-            const int q0 = c.ptr[i], len = c.ptr[i + 1] - q0;
-            if (len < 1 || len > W) { fits = false; continue; }
-            if (col)
-                for (int k = 0; k < stride; ++k) (*col)[(size_t)i * stride + k] = c.col[q0 + (k < len ? k : 0)];
-            const Csr &o = on ? *on : c;
-            for (int q = o.ptr[i]; q < o.ptr[i + 1]; ++q) {
-                int k = 0;
-                while (k < len && c.col[q0 + k] != o.col[q]) ++k;
-                if (k == len) { fits = false; break; }
-                val[(size_t)i * stride + k] = o.val[q];
-            }
-        }
-        return fits;
     };
     std::vector<int> col;
     std::vector<double> val;
@@ -2478,6 +2480,7 @@ namespace {
 // linearised step) with its block preconditioner and boundary columns
 struct BcSystem {
     DBuf col, val, a32, dinv, as64, as32, cpl64, cpl32;
+    DBuf bc7, bv7, be4, be4u;   // DevSolveOp::blk
     DevSolveOp op;
     ColsBufs bc[4];
     BcCols bcols;
@@ -2508,6 +2511,63 @@ BaroclinParams bc_params(const phg_bc_conf &c, double theta, bool backward) {
     bp.tau = c.tau; bp.sigma = c.sigma; bp.mu = c.mu; bp.sigma1 = c.sigma1; bp.mu1 = c.mu1;
     bp.alpha = c.alpha; bp.theta = theta; bp.backward = backward;
     return bp;
+}
+
+// the block system's parts for the persistent multigrid solver (DevSolveOp::blk):
+// A in block order (unknown q rs + i), dinv interleaved and scaled
+int build_bc_blk(phg_ops_s *o, const Csr &A, const std::vector<double> &dinv, double su, BcSystem &S) {
+    DevSolveOp &op = S.op;
+    op.mgx = o->L.op.mgx;
+    if (!op.mgx.nlev) return PHG_OK;
+    std::string err;
+    const MgHierarchy *h = o->mesh->hierarchy(err);
+    std::shared_ptr<const MgPlan> plan = h ? o->mesh->d->mg_plan(*h, op.mg.omega) : nullptr;
+    if (!plan) return PHG_OK;
+    const int rs = o->rs;
+    const Csr &M = o->mesh->ops.idt;
+    // the blocks' entries on the mass matrix's pattern
+    auto block = [&](int br, int bc) {
+        Csr B = M;
+        std::fill(B.val.begin(), B.val.end(), 0.0);
+        for (int i = 0; i < rs; ++i)
+            for (int q = A.ptr[br * rs + i]; q < A.ptr[br * rs + i + 1]; ++q) {
+                if (A.col[q] / rs != bc) continue;
+                const int *b = &M.col[M.ptr[i]], *e = b + (M.ptr[i + 1] - M.ptr[i]);
+                const int *at = std::lower_bound(b, e, A.col[q] % rs);
+                if (at != e && *at == A.col[q] % rs) B.val[M.ptr[i] + (at - b)] = A.val[q];
+            }
+        return B;
+    };
+    std::vector<int> col;
+    std::vector<double> val, v((size_t)6 * MGX_WT * rs);
+    for (int q = 0; q < 2; ++q) {
+        const Csr parts[3] = {M, block(0, q), block(1, q)};
+        for (int k = 0; k < 3; ++k) {
+            if (!rows_of(parts[k], nullptr, MGX_WT, MGX_WT, &col, val)) return PHG_OK;
+            for (int i = 0; i < rs; ++i)
+                for (int e = 0; e < MGX_WT; ++e)
+                    v[((size_t)i * 6 + 3 * q + k) * MGX_WT + e] = (k == 0 ? su : 1.0) * val[(size_t)i * MGX_WT + e] *
+                                                                 dinv[4 * (size_t)col[(size_t)i * MGX_WT + e] + q];
+        }
+    }
+    Csr e4 = block(1, 3);
+    for (double &x : e4.val) x = -x / su;
+    std::vector<double> v4, v4u;
+    if (!rows_of(plan->lev[0].T, &e4, MGX_WT, MGX_WT, nullptr, v4)) return PHG_OK;
+    const Csr e4u = csr_multiply(e4, plan->lev[0].U);
+    if (!rows_of(plan->AU, &e4u, MGX_WF, MGX_SF, nullptr, v4u)) return PHG_OK;
+    auto put = [&](DBuf &b, const std::vector<double> &x, const void **out) -> int {
+        if (o->prec == PHG_MIXED) CK(upload(b, to_f32(x)));
+        else CK(upload(b, x));
+        *out = b.p;
+        return PHG_OK;
+    };
+    int r;
+    if ((r = put(S.bv7, v, &op.blk.v)) || (r = put(S.be4, v4, &op.blk.e4)) || (r = put(S.be4u, v4u, &op.blk.e4u)))
+        return r;
+    CK(upload(S.bc7, col));
+    op.blk.c = S.bc7.as<int>();
+    return PHG_OK;
 }
 
 // assemble one 4rs block system, interleave it (unknown q*rs + i -> 4i + q),
@@ -2559,6 +2619,8 @@ int build_bc_system(phg_ops_s *o, const BaroclinParams &bp, double su, BcSystem 
         for (auto &x : mv) x *= su;
         CK(upload(S.cpl64, mv)); CK(upload(S.cpl32, to_f32(mv)));
         op.cpl = o->ell(S.cpl64); op.cpl32 = S.cpl32.as<float>();
+        const int r = build_bc_blk(o, A, dinv, su, S);
+        if (r) return r;
     } else {
         // small meshes (no multigrid hierarchy): Jacobi-scaled GMRES
         std::vector<double> as64(val.size());

@@ -102,7 +102,16 @@ struct DevSolveOp {
     const float *a32 = nullptr;    // A in FP32 (multigrid path, mixed precision)
     MgDev mg;                      // host copy (sizes)
     const MgDev *mgd = nullptr;    // the same descriptor in device memory (read by the kernel)
-    MgxDev mgx;                    // the V-cycle's composed operators
+    MgxDev mgx;                    // the V-cycle's composed operators (of L for a block system)
+    // A block system's parts on the finest level's pattern (rows of MGX_WT
+    // entries at c), in the handle's precision: per row and layer q three runs
+    // of MGX_WT values, all times 1 / diagonal of the layer's w rows -- the
+    // coupling M, and the entries of the w1 and w2 rows in layer q's w columns;
+    // e4, e4u: minus the w2 rows' u2 columns, and that times U (on F's pattern)
+    struct {
+        const int *c = nullptr;
+        const void *v = nullptr, *e4 = nullptr, *e4u = nullptr;
+    } blk;
     // Block preconditioner of a vertex-interleaved 4-field system (unknown
     // 4i+q, q = 0,1 "w" rows, q = 2,3 "u" rows whose diagonal blocks are -L):
     // z_w = D^-1 v_w, z_u = -Vcycle_L(v_u - M z_w); mgd is then the hierarchy

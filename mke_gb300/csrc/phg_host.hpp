@@ -116,6 +116,7 @@ struct MgPlan {
     std::vector<std::vector<double>> B;
     std::vector<double> E, AB, AE;
 };
+Csr csr_multiply(const Csr &A, const Csr &B);   // columns ascending
 bool build_mg_plan(const Csr &fine, const MgHierarchy &h, double omega, MgPlan &p);
 // BarVortex forward matrix c1 * mass + c2 * slaplace (examples/barvortex_impl.h:57-78)
 void assemble_barvortex(const Mesh &m, double c1, double c2, Csr &A, Csr &Abnd);

@@ -76,6 +76,8 @@ std::vector<double> multiply(const Csr &A, const std::vector<double> &B, int m) 
 
 }  // namespace
 
+Csr csr_multiply(const Csr &A, const Csr &B) { return multiply(A, B); }
+
 bool build_mg_plan(const Csr &fine, const MgHierarchy &h, double omega, MgPlan &p) {
     const int nlev = (int)h.A.size();
     p = MgPlan();

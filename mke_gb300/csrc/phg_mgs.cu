@@ -23,6 +23,14 @@
 //    the other warps are already in the next V-cycle.  The stopping test comes
 //    out of it too, so the last step's V-cycle is begun once in vain.
 //
+// The baroclinic block system (BLK; unknown 4i + q of vertex i, w1 w2 u1 u2) runs
+// through the same kernel: its preconditioner z_w = D^-1 v_w, z_u = -V(v_u - M z_w)
+// is one V-cycle of two vectors at once (C = 2, side by side), and its apply
+// needs no gather of z: the w rows' mass-like part comes with M z_w from the
+// gather of v, the u rows are M z_w - L z_u = M z_w + L V(t), which the
+// finest level's last gather gives as for one Laplacian, and u2's part of the
+// w2 rows is composed with it in the same way.
+//
 // Why no cell is overwritten too early: a block writes the cells of Arnoldi
 // step j + 1 only after it has collected the dot products of step j from every
 // block, and a block publishes its part of those after its own gathers of step
@@ -42,14 +50,14 @@ namespace {
 
 constexpr int RS = 33;           // stride of the warps' partial sums (up to 32 warps)
 constexpr int NB = 5;            // published sums a lane collects at a time
-constexpr int N_TAB = 3 * MG_MAXLEV + 1;
-enum { TAB_Q = 0, TAB_T = MG_MAXLEV, TAB_U = 2 * MG_MAXLEV, TAB_F = 3 * MG_MAXLEV };
+constexpr int N_TAB = 3 * MG_MAXLEV + 2;
+enum { TAB_Q = 0, TAB_T = MG_MAXLEV, TAB_U = 2 * MG_MAXLEV, TAB_F = 3 * MG_MAXLEV, TAB_C = 3 * MG_MAXLEV + 1 };
 
 // a sparse operator: entries and values of all rows in global memory, and the
 // shared-memory offsets of a block's own rows (off < 0: not copied)
 struct Table {
-    const void *c, *v, *v2;
-    int rows, off, off2, offc;
+    const void *c, *v, *v2, *v3;
+    int rows, off, off2, off3, offc;
 };
 // a block's rows of `words` 32-bit words each, copied to shared memory at dst
 struct Copy {
@@ -61,7 +69,8 @@ struct MgsParams {
     int x_n[MG_MAXLEV];        // rows of the levels
     const int *col;            // finest level: exact A (FP64 residuals)
     const double *aval;
-    int W, n, nv, ld, m, max_iter;
+    int W, n, nv, ld, m, max_iter;   // n: rows of the finest level (vertices of a block system)
+    const double *dinv;        // block system: 1 / diagonal
     double tol, inner_rtol;
     const double *B;
     double *X;
@@ -80,7 +89,7 @@ struct MgsParams {
     long long wait_limit;
     size_t boff[MG_MAXLEV], xoff[MG_MAXLEV];   // cell offsets of b_l and x_l (l >= 1)
     Table tab[N_TAB];
-    Copy copy[3 * N_TAB];
+    Copy copy[4 * N_TAB];
     int ncopy;
     const void *dense, *dense2;
     int off_d, off_d2;         // the dense rows in shared memory (-1: in global memory)
@@ -92,18 +101,18 @@ struct MgsParams {
 // this block's rows of one sparse operator: row i at c, v + (i - base) * stride
 template <typename VT> struct Rows {
     const int *c;
-    const VT *v, *v2;
+    const VT *v, *v2, *v3;
     int base;
 };
 
-// sum over N entries k = k0, k0 + KS, ... of row i: v[k] x[c[k]]
-template <typename VT, bool ONE, int N, int KS = 1>
+// sum over N entries of a row, KS apart: v[k] x[C c[k]] (C vectors side by side)
+template <typename VT, bool ONE, int N, int KS, int C>
 __device__ __forceinline__ VT row_sum(const int *col, const VT *v, const typename CellStore<VT, ONE>::E *p, unsigned stamp,
                                       const Waits &w) {
     int c[N];
     VT x[N];
 #pragma unroll
-    for (int q = 0; q < N; ++q) c[q] = col[KS * q];
+    for (int q = 0; q < N; ++q) c[q] = C * col[KS * q];
     CellStore<VT, ONE>::get(x, p, c, stamp, w);
     VT s = 0;
 #pragma unroll
@@ -156,10 +165,12 @@ __device__ __noinline__ VT root_sum(const Cell<VT> *part, int G, unsigned stamp,
     return warp_sum(s);
 }
 
-template <typename VT, bool ONE>
+// BLK: the block system of four unknowns per vertex (C = 2 vectors per V-cycle)
+template <typename VT, bool ONE, bool BLK>
 __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(const __grid_constant__ MgsParams p) {
     using ST = CellStore<VT, ONE>;
     using E = typename ST::E;
+    constexpr int C = BLK ? 2 : 1, NK = BLK ? 4 : 1;   // vectors per V-cycle, Krylov entries per finest row
     extern __shared__ __align__(16) char smem[];
     double *H = (double *)smem;              // (m + 1) x m, the R factor
     double *cs = H + (MAXM + 1) * MAXM, *sn = cs + MAXM, *g = sn + MAXM, *y = g + MAXM + 1;
@@ -198,7 +209,8 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
     const int *__restrict__ col = p.col;
     const double *__restrict__ aval = p.aval;
     E *cw = (E *)((char *)p.scratch + (size_t)grp * p.group_bytes);   // Krylov vector (not normalised)
-    E *ct = cw + n;                                                    // T b of the finest level
+    E *ct = cw + (size_t)NK * n;                                       // T b of the finest level
+    E *c0 = BLK ? ct + (size_t)C * n : cw;                             // b of the finest level
     E *cells = cw;
     VT *Vp = (VT *)p.V, *Zp = (VT *)p.Z;
     const double es = (double)sizeof(VT);
@@ -222,11 +234,12 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
     if (threadIdx.x < N_TAB) {
         const Table &t = p.tab[threadIdx.x];
         int i0 = 0, i1;
-        Rows<VT> A = {(const int *)t.c, (const VT *)t.v, (const VT *)t.v2, 0};
+        Rows<VT> A = {(const int *)t.c, (const VT *)t.v, (const VT *)t.v2, (const VT *)t.v3, 0};
         if (t.off >= 0) {
             own_rows(t.rows, G, bi, i0, i1);
             A.v = (const VT *)(smem + t.off);
             A.v2 = (const VT *)(smem + t.off2);
+            A.v3 = (const VT *)(smem + t.off3);
             A.c = (const int *)(smem + t.offc);
             A.base = i0;
         }
@@ -241,17 +254,23 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
     const VT *dn2 = p.off_d >= 0 ? (const VT *)(smem + p.off_d2) : (const VT *)p.dense2 + (size_t)d0 * nbs;
     VT *bsm = (VT *)(smem + p.off_b);
     VT *vsm = (VT *)(smem + p.off_v);
-    const int rpb = (n + G - 1) / G;
-    const int NA = max(1, min(NW, (r1 - r0 + 31) / 32));   // worker warps with rows of the finest level
+    const int rpb = NK * ((n + G - 1) / G), nk = NK * n;    // Krylov entries of a block, and in all
+    const int k0 = NK * r0, kn = NK * (r1 - r0);            // this block's
+    const int NA = max(1, min(NW, (kn + 31) / 32));         // worker warps with Krylov entries
     if (!ONE) {   // no stamp of an earlier launch survives (ordered by the first barrier below)
 #pragma unroll 1
-        for (int i = r0 + threadIdx.x; i < r1; i += blockDim.x) { ST::put(cw + i, (VT)0, 0u); ST::put(ct + i, (VT)0, 0u); }
+        for (int i = k0 + threadIdx.x; i < k0 + kn; i += blockDim.x) ST::put(cw + i, (VT)0, 0u);
+#pragma unroll 1
+        for (int i = C * r0 + threadIdx.x; i < C * r1; i += blockDim.x) {
+            ST::put(ct + i, (VT)0, 0u);
+            if (BLK) ST::put(c0 + i, (VT)0, 0u);
+        }
 #pragma unroll 1
         for (int l = 1; l <= bot; ++l) {
             int i0, i1;
             own_rows(p.x_n[l], G, bi, i0, i1);
 #pragma unroll 1
-            for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
+            for (int i = C * i0 + threadIdx.x; i < C * i1; i += blockDim.x) {
                 ST::put(cells + p.boff[l] + i, (VT)0, 0u);
                 ST::put(cells + p.xoff[l] + i, (VT)0, 0u);
             }
@@ -262,24 +281,25 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
             if (bi == 0) ST::put(csum + l, (VT)0, 0u);
         }
     }
-    for (int k = nb + threadIdx.x; k < nbs; k += blockDim.x) ((VT *)(smem + p.off_b))[k] = (VT)0;
+    for (int k = nb + threadIdx.x; k < nbs; k += blockDim.x)
+        for (int q = 0; q < C; ++q) bsm[q * nbs + k] = (VT)0;
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
 
     int my_iters = 0, my_cycles = 0, my_status = 0, my_steps = 0;
     double my_rel = 0.0, my_bytes = 0.0;
-    const double nrows = (double)(r1 - r0);
+    const double nrows = (double)kn;
     unsigned ep = 0;           // stamp of the current V-cycle
 
 #pragma unroll 1
     for (int v = grp; v < p.nv; v += p.groups) {
         const double *__restrict__ b = p.B + (size_t)v * ld;
         double *x = p.X + (size_t)v * ld;
-        VT *V = Vp + (size_t)v * (m + 1) * n, *Z = Zp + (size_t)v * m * n;
-        VT *wl = p.off_w >= 0 ? (VT *)(smem + p.off_w) : (VT *)p.Wv + (size_t)v * n + r0;   // own rows of A z
-        double *R = p.R + (size_t)v * n;
+        VT *V = Vp + (size_t)v * (m + 1) * nk, *Z = Zp + (size_t)v * m * nk;
+        VT *wl = p.off_w >= 0 ? (VT *)(smem + p.off_w) : (VT *)p.Wv + (size_t)v * nk + k0;   // own rows of A z
+        double *R = p.R + (size_t)v * nk;
         // own rows of Krylov vector l
-        auto vrow = [&](int l) -> VT * { return l < p.mv ? vsm + (size_t)l * rpb : V + (size_t)l * n + r0; };
+        auto vrow = [&](int l) -> VT * { return l < p.mv ? vsm + (size_t)l * rpb : V + (size_t)l * nk + k0; };
         int iters = 0, cycles = 0, status = 1;
         double beta_prev = 0.0, rel = 0.0, bnorm = 0.0;
 #pragma unroll 1
@@ -289,19 +309,25 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
                 double sb = 0.0, sr = 0.0;
                 if (!helper)
 #pragma unroll 1
-                    for (int i = r0 + threadIdx.x; i < r1; i += NW * 32) {
+                    for (int i = k0 + threadIdx.x; i < k0 + kn; i += NW * 32) {
                         double t = 0.0;
-                        int c[8];
-                        double a[8], xv[8];
+#pragma unroll 1
+                        for (int w0 = 0; w0 < W; w0 += 8) {
+                            int c[8];
+                            double a[8], xv[8];
 #pragma unroll
-                        for (int k = 0; k < 8; ++k)
-                            if (k < W) { c[k] = __ldg(&col[(size_t)k * n + i]); a[k] = __ldg(&aval[(size_t)k * n + i]); }
+                            for (int k = 0; k < 8; ++k)
+                                if (w0 + k < W) {
+                                    c[k] = __ldg(&col[(size_t)(w0 + k) * nk + i]);
+                                    a[k] = __ldg(&aval[(size_t)(w0 + k) * nk + i]);
+                                }
 #pragma unroll
-                        for (int k = 0; k < 8; ++k)
-                            if (k < W) xv[k] = ldcg(&x[c[k]]);
+                            for (int k = 0; k < 8; ++k)
+                                if (w0 + k < W) xv[k] = ldcg(&x[c[k]]);
 #pragma unroll
-                        for (int k = 0; k < 8; ++k)
-                            if (k < W) t += a[k] * xv[k];
+                            for (int k = 0; k < 8; ++k)
+                                if (w0 + k < W) t += a[k] * xv[k];
+                        }
                         const double bv = b[i], q = bv - t;
                         R[i] = q;
                         sr += q * q;
@@ -346,7 +372,7 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
             const double beta = scal[1];
             if (bnorm == 0.0) {
 #pragma unroll 1
-                for (int i = r0 + threadIdx.x; i < r1; i += blockDim.x) x[i] = 0.0;
+                for (int i = k0 + threadIdx.x; i < k0 + kn; i += blockDim.x) x[i] = 0.0;
                 status = 0; rel = 0.0;
                 break;
             }
@@ -361,10 +387,10 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
                 const double ib = scal[3];
                 VT *v0 = vrow(0);
 #pragma unroll 1
-                for (int i = r0 + threadIdx.x; i < r1; i += NW * 32) {
-                    const VT q = (VT)(R[i] * ib);
-                    v0[i - r0] = q;
-                    ST::put(cw + i, q, ep + 1);
+                for (int i = threadIdx.x; i < kn; i += NW * 32) {
+                    const VT q = (VT)(R[k0 + i] * ib);
+                    v0[i] = q;
+                    ST::put(cw + k0 + i, q, ep + 1);
                 }
             }
             if (ONE) __syncthreads();
@@ -413,61 +439,113 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
                         s_stop = 0;
                     }
                 }
+                const int tr = (C * (r1 - r0) + 31) / 32;   // warps' worth of the finest level's rows
+                if constexpr (BLK) {
+                    // t = v_u - M z_w with z_w = D^-1 v_w, and the w rows of A z
+                    // but for u2's part; lane pair = the two layers of a vertex
+                    if (!helper)
+#pragma unroll 1
+                        for (int t = warp; t < tr; t += NW) {
+                            const int it = t * 32 + lane, i = r0 + it / C, q = it % C, row = min(i, r1 - 1);
+                            const Rows<VT> &A = tab[TAB_C];
+                            const int *ce = A.c + (size_t)(row - A.base) * MGX_WT;
+                            const VT *ve = A.v + (size_t)(row - A.base) * (6 * MGX_WT) + q * (3 * MGX_WT);
+                            int c[MGX_WT + 2];
+                            VT u[MGX_WT + 2], sm = 0, s0 = 0, s1 = 0;
+#pragma unroll
+                            for (int k = 0; k < MGX_WT; ++k) c[k] = NK * ce[k] + q;
+                            c[MGX_WT] = NK * row + q;              // its own v_w and v_u
+                            c[MGX_WT + 1] = NK * row + 2 + q;
+                            ST::get(u, cw, c, ep, wt);
+#pragma unroll
+                            for (int k = 0; k < MGX_WT; ++k) {
+                                sm += ve[k] * u[k];
+                                s0 += ve[MGX_WT + k] * u[k];
+                                s1 += ve[2 * MGX_WT + k] * u[k];
+                            }
+                            s0 += __shfl_xor_sync(0xffffffffu, s0, 1);
+                            s1 += __shfl_xor_sync(0xffffffffu, s1, 1);
+                            if (i < r1) {
+                                const int e = NK * (i - r0) + q;
+                                ST::put(c0 + (size_t)C * i + q, u[MGX_WT + 1] - sm, ep);
+                                wl[e] = q ? s1 : s0;
+                                wl[e + 2] = sm;
+                                if (j < m) Z[(size_t)j * nk + k0 + e] = (VT)(p.dinv[k0 + e] * (double)u[MGX_WT]);
+                            }
+                        }
+                    if (ONE) __syncthreads();
+                }
+                // A times T b of the finest level (and u2's part of the w2 rows)
+                auto apply_tb = [&]() {
+#pragma unroll 1
+                    for (int t = warp; t < tr; t += NW) {
+                        const int it = t * 32 + lane, i = r0 + it / C, q = it % C;
+                        const Rows<VT> &A = tab[TAB_T];
+                        const size_t e = (size_t)(min(i, r1 - 1) - A.base) * MGX_WT;
+                        int c[MGX_WT];
+                        VT u[MGX_WT], s1 = 0, s2 = 0;
+#pragma unroll
+                        for (int k = 0; k < MGX_WT; ++k) c[k] = C * (A.c + e)[k] + q;
+                        ST::get(u, ct, c, ep, wt);
+#pragma unroll
+                        for (int k = 0; k < MGX_WT; ++k) {
+                            s1 += (A.v2 + e)[k] * u[k];
+                            if (BLK) s2 += (A.v3 + e)[k] * u[k];
+                        }
+                        if (i < r1) {
+                            if (BLK) {
+                                wl[NK * (i - r0) + 2 + q] += s1;
+                                if (q) wl[NK * (i - r0) + 1] += s2;
+                            } else {
+                                wl[i - r0] = s1;
+                            }
+                        }
+                    }
+                };
                 // down: b_{l+1} = Q_l b_l; T b of the finest level, and A times it one phase later
 #pragma unroll 1
                 for (int l = 0; l < bot; ++l) {
                     if (!helper) {
-                        const E *src = l == 0 ? cw : cells + p.boff[l];
+                        const E *src = l == 0 ? c0 : cells + p.boff[l];
                         E *dst = cells + p.boff[l + 1];
                         int i0, i1;
                         own_rows(p.x_n[l + 1], G, bi, i0, i1);
-                        const int tq = ((i1 - i0) * 4 + 31) / 32;        // four lanes per row of Q
-                        const int tr = l <= 1 ? (r1 - r0 + 31) / 32 : 0;
+                        const int tq = ((i1 - i0) * (4 * C) + 31) / 32;  // four lanes per row of Q (and vector)
 #pragma unroll 1
                         for (int t = warp; t < tq; t += NW) {
-                            const int q = t * 32 + lane, i = i0 + (q >> 2);
+                            const int q = t * 32 + lane, i = i0 + q / (4 * C), h = (q >> 2) % C;
                             const Rows<VT> &A = tab[TAB_Q + l];
                             const size_t e = (size_t)(min(i, i1 - 1) - A.base) * MGX_WQ + (q & 3);
-                            VT s = row_sum<VT, ONE, MGX_WQ / 4, 4>(A.c + e, A.v + e, src, ep, wt);
+                            VT s = row_sum<VT, ONE, MGX_WQ / 4, 4, C>(A.c + e, A.v + e, src + h, ep, wt);
                             s += __shfl_xor_sync(0xffffffffu, s, 1);
                             s += __shfl_xor_sync(0xffffffffu, s, 2);
-                            if (i < i1 && (q & 3) == 0) ST::put(dst + i, s, ep);
+                            if (i < i1 && (q & 3) == 0) ST::put(dst + (size_t)C * i + h, s, ep);
                         }
                         // the finest level's rows, by the same thread in every phase
+                        if (l == 0) {
 #pragma unroll 1
-                        for (int t = warp; t < tr; t += NW) {
-                            const int i = r0 + t * 32 + lane;
-                            const Rows<VT> &A = tab[TAB_T];
-                            const size_t e = (size_t)(min(i, r1 - 1) - A.base) * MGX_WT;
-                            if (l == 0) {
-                                const VT s = row_sum<VT, ONE, MGX_WT>(A.c + e, A.v + e, cw, ep, wt);
-                                if (i < r1) ST::put(ct + i, s, ep);
-                            } else {
-                                const VT s = row_sum<VT, ONE, MGX_WT>(A.c + e, A.v2 + e, ct, ep, wt);
-                                if (i < r1) wl[i - r0] = s;
+                            for (int t = warp; t < tr; t += NW) {
+                                const int it = t * 32 + lane, i = r0 + it / C, q = it % C;
+                                const Rows<VT> &A = tab[TAB_T];
+                                const size_t e = (size_t)(min(i, r1 - 1) - A.base) * MGX_WT;
+                                const VT s = row_sum<VT, ONE, MGX_WT, 1, C>(A.c + e, A.v + e, c0 + q, ep, wt);
+                                if (i < r1) ST::put(ct + (size_t)C * i + q, s, ep);
                             }
                         }
+                        if (l == 1) apply_tb();
                     }
                     if (ONE) __syncthreads();
                 }
-                if (bot == 1 && !helper)
-#pragma unroll 1
-                    for (int t = warp; t < (r1 - r0 + 31) / 32; t += NW) {
-                        const int i = r0 + t * 32 + lane;
-                        const Rows<VT> &A = tab[TAB_T];
-                        const size_t e = (size_t)(min(i, r1 - 1) - A.base) * MGX_WT;
-                        const VT s = row_sum<VT, ONE, MGX_WT>(A.c + e, A.v2 + e, ct, ep, wt);
-                        if (i < r1) wl[i - r0] = s;
-                    }
+                if (bot == 1 && !helper) apply_tb();
                 // dense: x_top = [T b +] E b_bot
                 if (!helper) {
-                    const E *src = bot == 0 ? cw : cells + p.boff[bot];
+                    const E *src = bot == 0 ? c0 : cells + p.boff[bot];
 #pragma unroll 1
-                    for (int q0 = warp * 32; q0 < nb; q0 += NW * 32) {
-                        const int c[1] = {min(q0 + lane, nb - 1)};
+                    for (int q0 = warp * 32; q0 < C * nb; q0 += NW * 32) {
+                        const int q = q0 + lane, c[1] = {min(q, C * nb - 1)};
                         VT t[1];
                         ST::get(t, src, c, ep, wt);
-                        if (q0 + lane < nb) bsm[q0 + lane] = t[0];
+                        if (q < C * nb) bsm[(q % C) * nbs + q / C] = t[0];
                     }
                 }
                 if (__syncthreads_or(s_dead)) return;
@@ -476,30 +554,31 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
                 const VT inv = (VT)s_inv;
                 if (!helper)
 #pragma unroll 1
-                    for (int i = d0 + warp; i < d1; i += NW) {
+                    for (int t = warp; t < C * (d1 - d0); t += NW) {
+                        const int i = d0 + t / C, h = t % C;
                         const VT *row = dn + (size_t)(i - d0) * nbs;
                         VT tb = 0;   // [T b] of the row
                         if (top == 0) {
                             if (bot > 0) {   // this block's own T b
                                 const int ci[1] = {i};
-                                VT t[1];
-                                ST::get(t, ct, ci, ep, wt);
-                                tb = t[0];
+                                VT t1[1];
+                                ST::get(t1, ct, ci, ep, wt);
+                                tb = t1[0];
                             }
                         } else if (top < bot) {   // level top = bot - 1
                             const Rows<VT> &A = tab[TAB_T + top];
                             const size_t e = (size_t)(i - A.base) * MGX_WT;
-                            tb = row_sum<VT, ONE, MGX_WT>(A.c + e, A.v + e, cells + p.boff[top], ep, wt);
+                            tb = row_sum<VT, ONE, MGX_WT, 1, C>(A.c + e, A.v + e, cells + p.boff[top] + h, ep, wt);
                         }
-                        const VT s = dense_row<VT>(row, bsm, nbs, lane) + tb;
-                        if (top > 0) {
-                            if (lane == 0) ST::put(cells + p.xoff[top] + i, s, ep);
+                        const VT s = dense_row<VT>(row, bsm + h * nbs, nbs, lane) + tb;
+                        if (BLK || top > 0) {
+                            if (lane == 0) ST::put(cells + p.xoff[top] + (size_t)C * i + h, s, ep);
                             continue;
                         }
                         VT s2 = dense_row<VT>(dn2 + (size_t)(i - d0) * nbs, bsm, nbs, lane);
                         if (lane == 0) {
                             if (bot > 0) s2 += wl[i - r0];
-                            Z[(size_t)j * n + i] = s * inv;
+                            Z[(size_t)j * nk + i] = s * inv;
                             wl[i - r0] = s2 * inv;
                             vrow(j)[i - r0] *= inv;
                         }
@@ -512,44 +591,56 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
                         int i0, i1;
                         own_rows(p.x_n[l], G, bi, i0, i1);
 #pragma unroll 1
-                        for (int t = warp; t < (i1 - i0 + 31) / 32; t += NW) {
-                            const int i = i0 + t * 32 + lane, row = min(i, i1 - 1);
+                        for (int t = warp; t < (C * (i1 - i0) + 31) / 32; t += NW) {
+                            const int it = t * 32 + lane, i = i0 + it / C, q = it % C, row = min(i, i1 - 1);
                             const Rows<VT> &A = tab[TAB_T + l], &U = tab[TAB_U + l];
                             const size_t e = (size_t)(row - A.base) * MGX_WT, f = (size_t)(row - U.base) * MGX_WU;
-                            VT s = row_sum<VT, ONE, MGX_WT>(A.c + e, A.v + e, cells + p.boff[l], ep, wt);
-                            s += row_sum<VT, ONE, MGX_WU>(U.c + f, U.v + f, cells + p.xoff[l + 1], ep, wt);
-                            if (i < i1) ST::put(cells + p.xoff[l] + i, s, ep);
+                            VT s = row_sum<VT, ONE, MGX_WT, 1, C>(A.c + e, A.v + e, cells + p.boff[l] + q, ep, wt);
+                            s += row_sum<VT, ONE, MGX_WU, 1, C>(U.c + f, U.v + f, cells + p.xoff[l + 1] + q, ep, wt);
+                            if (i < i1) ST::put(cells + p.xoff[l] + (size_t)C * i + q, s, ep);
                         }
                     }
                     if (ONE) __syncthreads();
                 }
                 // finest level: z = T b + U x_1 and A z = A T b + A U x_1, normalised
-                if (top > 0 && !helper)
+                if ((BLK || top > 0) && !helper)
 #pragma unroll 1
-                    for (int t = warp; t < (r1 - r0 + 31) / 32; t += NW) {
-                        const int i = r0 + t * 32 + lane, row = min(i, r1 - 1);
+                    for (int t = warp; t < tr; t += NW) {
+                        const int it = t * 32 + lane, i = r0 + it / C, h = it % C, row = min(i, r1 - 1);
                         const Rows<VT> &F = tab[TAB_F];
                         const size_t e = (size_t)(row - F.base) * MGX_SF;
-                        const int ci[1] = {row};
+                        const int ci[1] = {C * row + h};
                         int c[MGX_WF];
                         VT tb[1], x1[MGX_WF];
 #pragma unroll
-                        for (int q = 0; q < MGX_WF; ++q) c[q] = (F.c + e)[q];
+                        for (int q = 0; q < MGX_WF; ++q) c[q] = C * (F.c + e)[q] + h;
                         ST::get(tb, ct, ci, ep, wt);   // this block's own T b
                         ST::get(x1, cells + p.xoff[1], c, ep, wt);
-                        VT s = 0, aw = 0;
+                        VT s = 0, aw = 0, ew = 0;
 #pragma unroll
                         for (int q = 0; q < MGX_WF; ++q) {
                             s += (F.v + e)[q] * x1[q];
                             aw += (F.v2 + e)[q] * x1[q];
+                            if (BLK) ew += (F.v3 + e)[q] * x1[q];
                         }
                         if (i < r1) {
-                            const int q = i - r0;
-                            Z[(size_t)j * n + i] = (tb[0] + s) * inv;
-                            wl[q] = (wl[q] + aw) * inv;
-                            vrow(j)[q] *= inv;
+                            const int q = NK * (i - r0) + h;
+                            VT *vj = vrow(j), *zj = Z + (size_t)j * nk + k0;
+                            if (BLK) {
+                                zj[q] *= inv;
+                                zj[q + 2] = -(tb[0] + s) * inv;
+                                wl[q] = (h ? wl[q] + ew : wl[q]) * inv;
+                                wl[q + 2] = (wl[q + 2] + aw) * inv;
+                                vj[q] *= inv;
+                                vj[q + 2] *= inv;
+                            } else {
+                                zj[q] = (tb[0] + s) * inv;
+                                wl[q] = (wl[q] + aw) * inv;
+                                vj[q] *= inv;
+                            }
                         }
                     }
+                if (BLK) __syncthreads();   // the vectors' entries change hands
                 my_bytes += nrows * (p.step_row_bytes + es * 2.0 * (j + 1));
                 // dots with v_0..v_j, eight basis vectors per pass, on this thread's own rows
                 if (warp < NA)
@@ -560,7 +651,7 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
                         if (l0 + 8 <= p.mvp) {   // all in shared memory (those past j: not used)
                             const VT *v0 = vsm + l0 * rpb;
 #pragma unroll 1
-                            for (int q = threadIdx.x; q < r1 - r0; q += NW * 32) {
+                            for (int q = threadIdx.x; q < kn; q += NW * 32) {
                                 const VT s = wl[q];
 #pragma unroll
                                 for (int k = 0; k < 8; ++k) t[k] += v0[k * rpb + q] * s;
@@ -570,7 +661,7 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
 #pragma unroll
                             for (int k = 0; k < 8; ++k) vp[k] = vrow(l0 + (k < kk ? k : 0));
 #pragma unroll 1
-                            for (int q = threadIdx.x; q < r1 - r0; q += NW * 32) {
+                            for (int q = threadIdx.x; q < kn; q += NW * 32) {
                                 const VT s = wl[q];
 #pragma unroll
                                 for (int k = 0; k < 8; ++k) t[k] += vp[k][q] * s;
@@ -622,7 +713,7 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
                     VT a2 = 0;
                     VT *vn = vrow(j + 1);
 #pragma unroll 1
-                    for (int q = threadIdx.x; q < r1 - r0; q += NW * 32) {
+                    for (int q = threadIdx.x; q < kn; q += NW * 32) {
                         VT s = wl[q];
 #pragma unroll 1
                         for (int l0 = 0; l0 <= j; l0 += 8) {
@@ -642,7 +733,7 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
                             }
                         }
                         vn[q] = s;
-                        ST::put(cw + r0 + q, s, ep + 1);
+                        ST::put(cw + k0 + q, s, ep + 1);
                         a2 += s * s;
                     }
                     if (warp < NA) {
@@ -677,10 +768,10 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
             __syncthreads();
             if (!helper)
 #pragma unroll 1
-                for (int i = r0 + threadIdx.x; i < r1; i += NW * 32) {
+                for (int i = k0 + threadIdx.x; i < k0 + kn; i += NW * 32) {
                     VT s = 0;
 #pragma unroll 8
-                    for (int l = 0; l < jl; ++l) s += hv[l] * Z[(size_t)l * n + i];
+                    for (int l = 0; l < jl; ++l) s += hv[l] * Z[(size_t)l * nk + i];
                     x[i] += (double)s;
                 }
             my_bytes += nrows * (jl * es + 24.0);
@@ -713,25 +804,28 @@ size_t mgs_fixed_smem() {
            sizeof(double) * (MAXM + 2);
 }
 
-void *mgs_fn(Precision prec, bool one) {
-    return prec == PREC_MIXED ? (one ? (void *)mgs_kernel<float, true> : (void *)mgs_kernel<float, false>)
-                              : (one ? (void *)mgs_kernel<double, true> : (void *)mgs_kernel<double, false>);
+void *mgs_fn(Precision prec, int kind) {   // kind 0: blocks share right-hand sides, 1: a block each, 2: block system
+    if (prec == PREC_MIXED)
+        return kind == 0 ? (void *)mgs_kernel<float, false, false>
+             : kind == 1 ? (void *)mgs_kernel<float, true, false> : (void *)mgs_kernel<float, false, true>;
+    return kind == 0 ? (void *)mgs_kernel<double, false, false>
+         : kind == 1 ? (void *)mgs_kernel<double, true, false> : (void *)mgs_kernel<double, false, true>;
 }
 
 // bytes of dynamic shared memory a block may take (set once per kernel)
-cudaError_t mgs_smem_limit(Precision prec, bool one, int *limit) {
-    static std::once_flag once[4];
-    static cudaError_t err[4];
-    static int lim[4];
-    const int k = (prec == PREC_MIXED ? 1 : 0) + (one ? 2 : 0);
+cudaError_t mgs_smem_limit(Precision prec, int kind, int *limit) {
+    static std::once_flag once[6];
+    static cudaError_t err[6];
+    static int lim[6];
+    const int k = (prec == PREC_MIXED ? 1 : 0) + 2 * kind;
     std::call_once(once[k], [&] {
         int dev = 0, optin = 0;
         cudaFuncAttributes fa;
         if ((err[k] = cudaGetDevice(&dev)) != cudaSuccess) return;
         if ((err[k] = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess) return;
-        if ((err[k] = cudaFuncGetAttributes(&fa, mgs_fn(prec, one))) != cudaSuccess) return;
+        if ((err[k] = cudaFuncGetAttributes(&fa, mgs_fn(prec, kind))) != cudaSuccess) return;
         lim[k] = optin - (int)fa.sharedSizeBytes;
-        err[k] = cudaFuncSetAttribute(mgs_fn(prec, one), cudaFuncAttributeMaxDynamicSharedMemorySize, lim[k]);
+        err[k] = cudaFuncSetAttribute(mgs_fn(prec, kind), cudaFuncAttributeMaxDynamicSharedMemorySize, lim[k]);
     });
     *limit = lim[k];
     return err[k];
@@ -741,18 +835,21 @@ cudaError_t mgs_smem_limit(Precision prec, bool one, int *limit) {
 
 size_t mgs_scratch_bytes(const DevSolveOp &op, Precision prec) {
     const size_t cell = prec == PREC_MIXED ? 8 : 16;
-    size_t cells = 2 * (size_t)op.A.n;
-    for (int l = 1; l < op.mgx.nlev; ++l) cells += 2 * (size_t)op.mgx.lev[l].n;
+    const size_t C = op.block4 ? 2 : 1, n = (size_t)op.mgx.lev[0].n;
+    size_t cells = op.block4 ? 8 * n : 2 * n;
+    for (int l = 1; l < op.mgx.nlev; ++l) cells += 2 * C * op.mgx.lev[l].n;
     return (cells * cell + 255) & ~size_t(255);
 }
 
 bool mgs_applicable(const DevSolveOp &op) {
-    return op.mgx.nlev >= 2 && !op.block4 && op.A.W <= 8;
+    return op.mgx.nlev >= 2 && (op.block4 ? op.blk.c != nullptr : op.A.W <= 8);
 }
 
 cudaError_t mgs_solve(const DevSolveOp &op, const MgsArgs &q, cudaStream_t s) {
     const MgxDev &x = op.mgx;
-    const int n = op.A.n, nlev = x.nlev;
+    const bool blk = op.block4 != 0;
+    const size_t C = blk ? 2 : 1, NK = blk ? 4 : 1;
+    const int n = x.lev[0].n, nlev = x.nlev;
     const bool mixed = q.prec == PREC_MIXED;
     const size_t es = mixed ? 4 : 8;
     const int sms = (q.max_sms > 0 && q.max_sms < q.sms) ? q.max_sms : q.sms;
@@ -769,9 +866,9 @@ cudaError_t mgs_solve(const DevSolveOp &op, const MgsArgs &q, cudaStream_t s) {
     int G = cap / groups;
     if (q.rpb > 0) G = std::min(G, (n + q.rpb - 1) / q.rpb);
     G = std::max(G, 1);
-    const bool one = G == 1;
+    const bool one = G == 1 && !blk;
     int limit = 0;
-    cudaError_t e = mgs_smem_limit(q.prec, one, &limit);
+    cudaError_t e = mgs_smem_limit(q.prec, blk ? 2 : one ? 1 : 0, &limit);
     if (e != cudaSuccess) return e;
     size_t budget = (size_t)limit;
     if (many) budget = std::min<size_t>(budget, 104 * 1024);
@@ -788,7 +885,7 @@ cudaError_t mgs_solve(const DevSolveOp &op, const MgsArgs &q, cudaStream_t s) {
         for (int wide = 0; wide < 2; ++wide) {
             const int top = k - wide;
             if (wide && (k != x.first_dense || !x.E)) continue;
-            if (top == 0 && !(wide ? x.AE : x.AB)) continue;
+            if (top == 0 && (blk || !(wide ? x.AE : x.AB))) continue;
             const double rows = (double)((x.lev[top].n + G - 1) / G), ent = rows * x.lev[k].n * (top == 0 ? 2.0 : 1.0);
             const bool cached = mgs_fixed_smem() + es * ent < 0.6 * (double)budget;
             const double rate = mixed ? (cached ? 48.0 : 14.0) : (cached ? 1.6 : 1.5);
@@ -807,30 +904,36 @@ cudaError_t mgs_solve(const DevSolveOp &op, const MgsArgs &q, cudaStream_t s) {
         return o;
     };
     auto rpb = [&](int l) { return (size_t)((x.lev[l].n + G - 1) / G); };
-    p.off_b = take(es * (size_t)mgx_stride(x.lev[p.bot].n));
+    p.off_b = take(C * es * (size_t)mgx_stride(x.lev[p.bot].n));
     if (p.off_b < 0) return cudaErrorInvalidValue;
-    p.off_w = take(es * rpb(0));
+    p.off_w = take(NK * es * rpb(0));
     auto copy = [&](const void *src, int rows, int words, int dst) {
         Copy &c = p.copy[p.ncopy++];
         c.src = src; c.rows = rows; c.words = words; c.dst = dst;
     };
-    auto table = [&](int t, const int *c, const void *v, const void *v2, int rows, size_t rows_b, int width) {
+    // one to three value arrays of vw values a row on a pattern of `width` entries
+    auto table = [&](int t, const int *c, const void *v, const void *v2, const void *v3, int rows, size_t rows_b,
+                     int width, int vw) {
         Table &T = p.tab[t];
-        T.c = c; T.v = v; T.v2 = v2; T.rows = rows;
-        const size_t vb = (rows_b * width * es + 15) & ~size_t(15);
-        T.off = take((v2 ? 2 : 1) * vb + rows_b * width * 4);
+        T.c = c; T.v = v; T.v2 = v2; T.v3 = v3; T.rows = rows;
+        const size_t vb = (rows_b * vw * es + 15) & ~size_t(15);
+        const int arrays = v3 ? 3 : v2 ? 2 : 1;
+        T.off = take(arrays * vb + rows_b * width * 4);
         if (T.off < 0) return;
         T.off2 = T.off + (int)vb;
-        T.offc = T.off + (int)((v2 ? 2 : 1) * vb);
-        copy(v, rows, width * (int)es / 4, T.off);
-        if (v2) copy(v2, rows, width * (int)es / 4, T.off2);
+        T.off3 = T.off2 + (int)vb;
+        T.offc = T.off + arrays * (int)vb;
+        copy(v, rows, vw * (int)es / 4, T.off);
+        if (v2) copy(v2, rows, vw * (int)es / 4, T.off2);
+        if (v3) copy(v3, rows, vw * (int)es / 4, T.off3);
         copy(c, rows, width, T.offc);
     };
     for (int t = 0; t < N_TAB; ++t) p.tab[t].off = -1;
     for (int l = p.bot - 1; l >= 1; --l) {
-        table(TAB_T + l, x.lev[l].tc, x.lev[l].tv, nullptr, x.lev[l].n, rpb(l), MGX_WT);
-        table(TAB_Q + l, x.lev[l].qc, x.lev[l].qv, nullptr, x.lev[l + 1].n, rpb(l + 1), MGX_WQ);
-        if (l < p.top) table(TAB_U + l, x.lev[l].uc, x.lev[l].uv, nullptr, x.lev[l].n, rpb(l), MGX_WU);
+        table(TAB_T + l, x.lev[l].tc, x.lev[l].tv, nullptr, nullptr, x.lev[l].n, rpb(l), MGX_WT, MGX_WT);
+        table(TAB_Q + l, x.lev[l].qc, x.lev[l].qv, nullptr, nullptr, x.lev[l + 1].n, rpb(l + 1), MGX_WQ, MGX_WQ);
+        if (l < p.top)
+            table(TAB_U + l, x.lev[l].uc, x.lev[l].uv, nullptr, nullptr, x.lev[l].n, rpb(l), MGX_WU, MGX_WU);
     }
     p.dense = p.top < p.bot ? x.E : x.B[p.bot];
     p.dense2 = p.top == 0 ? (p.bot == 0 ? x.AB : x.AE) : nullptr;
@@ -845,17 +948,18 @@ cudaError_t mgs_solve(const DevSolveOp &op, const MgsArgs &q, cudaStream_t s) {
         }
     }
     if (p.bot > 0) {
-        table(TAB_T, x.lev[0].tc, x.lev[0].tv, x.a, n, rpb(0), MGX_WT);
-        table(TAB_Q, x.lev[0].qc, x.lev[0].qv, nullptr, x.lev[1].n, rpb(1), MGX_WQ);
+        table(TAB_T, x.lev[0].tc, x.lev[0].tv, x.a, blk ? op.blk.e4 : nullptr, n, rpb(0), MGX_WT, MGX_WT);
+        table(TAB_Q, x.lev[0].qc, x.lev[0].qv, nullptr, nullptr, x.lev[1].n, rpb(1), MGX_WQ, MGX_WQ);
     }
-    if (p.top > 0) table(TAB_F, x.fc, x.fu, x.fa, n, rpb(0), MGX_SF);
+    if (p.top > 0) table(TAB_F, x.fc, x.fu, x.fa, blk ? op.blk.e4u : nullptr, n, rpb(0), MGX_SF, MGX_SF);
+    if (blk) table(TAB_C, op.blk.c, op.blk.v, nullptr, nullptr, n, rpb(0), MGX_WT, 6 * MGX_WT);
     p.off_v = (int)used;
     // whole batches of eight, also past the last vector
-    p.mvp = (int)std::min<size_t>((q.m + 8) / 8 * 8, (budget - used) / (es * rpb(0)) / 8 * 8);
+    p.mvp = (int)std::min<size_t>((q.m + 8) / 8 * 8, (budget - used) / (NK * es * rpb(0)) / 8 * 8);
     p.mv = std::min(p.mvp, q.m + 1);
-    used += (size_t)p.mvp * es * rpb(0);
+    used += (size_t)p.mvp * NK * es * rpb(0);
 
-    p.col = op.A.col; p.aval = op.A.val;
+    p.col = op.A.col; p.aval = op.A.val; p.dinv = op.dinv;
     p.W = op.A.W; p.n = n; p.nv = q.nv; p.ld = q.ld; p.m = q.m; p.max_iter = q.max_iter;
     p.tol = q.tol; p.inner_rtol = q.inner_rtol;
     p.B = q.B; p.X = q.X;
@@ -868,8 +972,8 @@ cudaError_t mgs_solve(const DevSolveOp &op, const MgsArgs &q, cudaStream_t s) {
     p.bar = q.bar; p.err = q.err; p.stats = q.stats;
     p.groups = groups; p.G = G;
     p.wait_limit = q.wait_limit;
-    size_t c = 2 * (size_t)n;
-    for (int l = 1; l < nlev; ++l) { p.boff[l] = c; c += x.lev[l].n; p.xoff[l] = c; c += x.lev[l].n; }
+    size_t c = (blk ? 8 : 2) * (size_t)n;
+    for (int l = 1; l < nlev; ++l) { p.boff[l] = c; c += C * x.lev[l].n; p.xoff[l] = c; c += C * x.lev[l].n; }
     // algorithmic bytes per finest row: the residual, and one Arnoldi step
     // (operators once, each level's vectors once in and once out, w and v)
     p.resid_row_bytes = op.A.W * 12.0 + 24.0;
@@ -882,6 +986,8 @@ cudaError_t mgs_solve(const DevSolveOp &op, const MgsArgs &q, cudaStream_t s) {
     if (p.bot > 0) p.step_row_bytes += op.A.W * es;
     if (p.top > 0) p.step_row_bytes += MGX_WF * (4.0 + 2.0 * es);
     p.step_row_bytes += (double)x.lev[p.top].n * x.lev[p.bot].n * es / n * (p.top == 0 ? 2.0 : 1.0);
+    // per Krylov entry of a block system: four per finest row, the matrices read once for both vectors
+    if (blk) p.step_row_bytes = p.step_row_bytes / 4.0 + 7.0 * (4.0 + 6.0 * es) / 4.0 + 6.0 * es;
 
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute coop[1];
@@ -894,7 +1000,7 @@ cudaError_t mgs_solve(const DevSolveOp &op, const MgsArgs &q, cudaStream_t s) {
     cfg.attrs = coop;
     cfg.numAttrs = 1;
     void *args[] = {&p};
-    if ((e = cudaLaunchKernelExC(&cfg, mgs_fn(q.prec, one), args)) != cudaSuccess) return e;
+    if ((e = cudaLaunchKernelExC(&cfg, mgs_fn(q.prec, blk ? 2 : one ? 1 : 0), args)) != cudaSuccess) return e;
     mgs_fold_err<<<1, 1, 0, s>>>(q.err, q.stats);
     g_kernel_launches += 2;
     return cudaGetLastError();
