@@ -538,7 +538,7 @@ struct phg_ops_s {
     int max_sms = 0;                 // SMs the persistent solver may fill (0 = all)
     long long wait_limit = 0;        // barrier wait limit of the persistent solvers (0 = default ~1 s)
     // scratch
-    DBuf work, stats, s_a, s_b, s_c, s_d, s_e, s_part, s_out;
+    DBuf work, stats, s_a, s_b, s_c, s_e, s_part, s_out;
     GmresStats last{};
     bool stats_pending = false;
     int pending_slots = 0;           // stats slots written since the last check
@@ -1181,20 +1181,8 @@ int jacobian_derivs_dev(phg_ops_s *o, const double *u, const double *v, int ld, 
 
 int norm_dev(phg_ops_s *o, const double *u, const double *v, int nv, double *out_dev, bool dist, bool take_sqrt,
              cudaStream_t s) {
-    const int V = o->V;
-    CK(o->s_d.ensure(8 * (size_t)V * nv * 2));
-    double *diff = o->s_d.as<double>(), *y = diff + (size_t)V * nv;
-    const double *x = u;
-    if (dist) { CK(vsub(diff, u, v, (long long)V * nv, s)); x = diff; }
-    CK(apply_op(o->norm, DevCols(), x, V, nullptr, nullptr, 0, nullptr, y, V, nv, s));
-    CK(o->s_part.ensure(8 * (size_t)nv * dot_chunks(V)));
-    const double *a = dist ? x : u;
-    const double *bb = dist ? y : y;
-    if (!dist && v) {  // scalar(u, v) = u . (NORM v)
-        CK(apply_op(o->norm, DevCols(), v, V, nullptr, nullptr, 0, nullptr, y, V, nv, s));
-        a = u;
-    }
-    CK(dot(a, bb, V, V, nv, o->s_part.as<double>(), out_dev, take_sqrt, s));
+    CK(o->s_part.ensure(8 * (size_t)nv * norm_chunks(o->V)));
+    CK(norm_dot(o->norm, u, v ? v : u, dist, nv, o->s_part.as<double>(), out_dev, take_sqrt, s));
     return PHG_OK;
 }
 
@@ -1873,7 +1861,7 @@ struct phg_barvortex_s {
     ColsBufs Ab;
     DBuf lh;
     int cap = 0;   // members the buffers hold
-    DBuf w, dw, FC, u_n, w_n, u_n1, tmp1, tmp2, uin, F, rp, x, jsol, nr0, nr, done, ubnd, wbnd, frc;
+    DBuf w, dw, FC, u_n, w_n, u_n1, tmp1, tmp2, uin, F, rp, x, xu, jsol, nr0, nr, done, ubnd, wbnd, frc;
     std::vector<GmresStats> each;   // the last step's solve records, one per slot
     int nslots = 0;
     cudaStream_t last_stream = nullptr;   // stream of the last step (its stats live there)
@@ -1972,7 +1960,7 @@ int bv_reserve(phg_barvortex_s *b, int nv) {
     const size_t V = b->o->V, rs = b->o->rs, os = std::max(1, b->o->os);
     DBuf *full[] = {&b->w, &b->dw, &b->FC, &b->u_n, &b->w_n, &b->u_n1, &b->tmp1, &b->tmp2, &b->uin};
     for (DBuf *d : full) CK(d->ensure(8 * V * nv));
-    DBuf *inner[] = {&b->F, &b->rp, &b->x};
+    DBuf *inner[] = {&b->F, &b->rp, &b->x, &b->xu};
     for (DBuf *d : inner) CK(d->ensure(8 * rs * nv));
     CK(b->jsol.ensure(8 * rs * 8 * nv));
     CK(b->nr0.ensure(8 * nv)); CK(b->nr.ensure(8 * nv)); CK(b->done.ensure(4 * nv));
@@ -1994,7 +1982,7 @@ int bv_step_dev(phg_barvortex_s *b, int nv, double *u1, const double *u, const d
     double *w = b->w.as<double>(), *dw = b->dw.as<double>(), *FC = b->FC.as<double>();
     double *u_n = b->u_n.as<double>(), *w_n = b->w_n.as<double>(), *u_n1 = b->u_n1.as<double>();
     double *tmp1 = b->tmp1.as<double>(), *tmp2 = b->tmp2.as<double>(), *uu = b->uin.as<double>();
-    double *F = b->F.as<double>(), *rp = b->rp.as<double>(), *x = b->x.as<double>();
+    double *F = b->F.as<double>(), *rp = b->rp.as<double>(), *x = b->x.as<double>(), *xu = b->xu.as<double>();
     double *jsol = b->jsol.as<double>();
     const int *p2io = o->p2io.as<int>(), *isb = o->isb.as<int>();
     // keep the input: u1 may alias u
@@ -2020,15 +2008,15 @@ int bv_step_dev(phg_barvortex_s *b, int nv, double *u1, const double *u, const d
         CK(jac_combine(jsol, rs, rs, F, rs, FC, V, o->imap(), nv, s));
         // rp = M_L F + bnd_ bnd_w ; w_n = p2u(A^-1 rp, bnd_w)
         CK(apply_op(o->ML.op.A, b->Ab.c, F, rs, nullptr, bnd_w, os, nullptr, rp, rs, nv, s));
-        // warm start: previous w_n (first iteration: w), inner part
-        CK(gather(x, rs, it == 0 ? w : w_n, V, o->imap(), rs, nv, s));
+        // warm start from the previous iterate, which x holds (the first time: w);
+        // likewise xu for the Laplacian (u)
+        if (it == 0) CK(gather(x, rs, w, V, o->imap(), rs, nv, s));
         if ((r = solve(o, b->A.op, rp, x, nv, rs, o->tol, slot++, s))) return r;
-        CK(p2u(w_n, V, x, rs, bnd_w, os, p2io, isb, V, nv, s));
-        // u_n1 = Laplace^-1(w_n) with bnd_u: b = M_L w_n_in + B2 bnd_u
-        CK(apply_op(o->ML.op.A, o->bnd2.c, w_n, V, o->imap(), bnd_u, os, nullptr, rp, rs, nv, s));
-        CK(gather(x, rs, it == 0 ? uu : u_n, V, o->imap(), rs, nv, s));
-        if ((r = solve(o, o->L.op, rp, x, nv, rs, o->tol, slot++, s))) return r;
-        CK(p2u(u_n1, V, x, rs, bnd_u, os, p2io, isb, V, nv, s));
+        // w_n = p2u(x, bnd_w); u_n1 = Laplace^-1(w_n) with bnd_u: b = M_L w_n_in + B2 bnd_u
+        CK(p2u_apply(w_n, x, bnd_w, os, p2io, isb, V, o->ML.op.A, o->bnd2.c, bnd_u, rp, nv, s));
+        if (it == 0) CK(gather(xu, rs, uu, V, o->imap(), rs, nv, s));
+        if ((r = solve(o, o->L.op, rp, xu, nv, rs, o->tol, slot++, s))) return r;
+        CK(p2u(u_n1, V, xu, rs, bnd_u, os, p2io, isb, V, nv, s));
         // nr = dist(u_n1, u_n); u_n <- u_n1; stop test
         if ((r = norm_dev(o, u_n1, u_n, nv, b->nr.as<double>(), true, true, s))) return r;
         CK(bv_commit(u_n, u_n1, b->nr.as<double>(), b->nr0.as<double>(), b->done.as<int>(), V, nv, s));
@@ -2116,12 +2104,12 @@ static unsigned long long bv_sig(const phg_barvortex_s *b) {
     word(tb);
     word((unsigned long long)o->wait_limit);
     word((unsigned long long)o->jq_mode);
-    for (const DBuf *d : {&o->work, &o->stats, &o->s_a, &o->s_b, &o->s_c, &o->s_d, &o->s_e, &o->s_part, &o->s_out,
+    for (const DBuf *d : {&o->work, &o->stats, &o->s_a, &o->s_b, &o->s_c, &o->s_e, &o->s_part, &o->s_out,
                           &o->jq_split, &o->hist})
         mix(*d);
     for (const DBuf &d : o->st) mix(d);
     for (const DBuf *d : {&b->w, &b->dw, &b->FC, &b->u_n, &b->w_n, &b->u_n1, &b->tmp1, &b->tmp2, &b->uin, &b->F,
-                          &b->rp, &b->x, &b->jsol, &b->nr0, &b->nr, &b->done, &b->ubnd, &b->wbnd, &b->frc, &b->agg})
+                          &b->rp, &b->x, &b->xu, &b->jsol, &b->nr0, &b->nr, &b->done, &b->ubnd, &b->wbnd, &b->frc, &b->agg})
         mix(*d);
     return h;
 }

@@ -29,9 +29,8 @@ struct ChsArgs {
     void *work;            // chs_work_bytes
     double *R;             // nv x n
     double *part;          // partial sums of the blocks
-    unsigned *bar;         // zeroed with err before the launch
-    int *err;
-    GmresStats *stats;     // zeroed before the launch
+    unsigned *bar;         // zeroed before the launch
+    GmresStats *stats;     // zeroed before the launch; its status is the launch's error flag
 };
 
 size_t chs_work_bytes(const DevSolveOp &op, int nv, Precision prec, int sms);

@@ -435,7 +435,7 @@ __device__ __forceinline__ bool tail_enter(unsigned long long *ccnt, int CS, int
                         v = prev;
                     }
                     g = (v & CCNT_POISON) ? 0 : 1;
-                    if (!g) atomicExch(err, 1);
+                    if (!g) atomicMax(err, STATUS_TIMEOUT);
                     break;
                 }
             }
@@ -1215,15 +1215,11 @@ __global__ void __launch_bounds__(BLOCK, 2) cheb_kernel(const Params p) {
     }
 }
 
-__global__ void fold_err(const int *err, GmresStats *st) {
-    if (*err) st->status = 2;
-}
-
 size_t smem_gmres_bytes() { return sizeof(double) * ((MAXM + 1) * MAXM + 2 * MAXM + (MAXM + 1) + MAXM + (MAXM + 2)); }
 
 constexpr int GROUPS_CAP = 4096;
 
-struct Layout { size_t v, z, w, r, mg, part, bar, err, ccnt, total; };
+struct Layout { size_t v, z, w, r, mg, part, bar, ccnt, total; };
 
 // per-group multigrid scratch: one V-cycle's levels, or two V-cycles' levels
 // and the 4 vertex vectors of the block preconditioner
@@ -1269,8 +1265,7 @@ Layout layout(const DevSolveOp &op, int nv, int m, Precision prec) {
     L.part = L.mg + (mg ? al(gb * (size_t)groups) : 0);
     // groups * G <= co-resident blocks (< 4096)
     L.bar = L.part + al(8 * (size_t)4096 * 2 * (MAXM + 2));
-    L.err = L.bar + al(8 * (size_t)GROUPS_CAP);
-    L.ccnt = L.err + 256;
+    L.ccnt = L.bar + al(8 * (size_t)GROUPS_CAP);
     L.total = L.ccnt + al(8 * (size_t)GROUPS_CAP);
     return L;
 }
@@ -2608,7 +2603,7 @@ cudaError_t gmres_solve(const DevSolveOp &op, const double *B, double *X, int nv
         const Layout L = layout(op, nv, m, prec);
         char *w = (char *)work;
         cudaError_t e0;
-        if ((e0 = cudaMemsetAsync(w + L.bar, 0, L.total - L.bar, s)) != cudaSuccess) return e0;
+        if ((e0 = cudaMemsetAsync(w + L.bar, 0, L.ccnt - L.bar, s)) != cudaSuccess) return e0;
         if ((e0 = cudaMemsetAsync(stats_dev, 0, sizeof(GmresStats), s)) != cudaSuccess) return e0;
         const char *ev = getenv("PHG_INNER_RTOL");
         ChebPlan pl;
@@ -2618,14 +2613,14 @@ cudaError_t gmres_solve(const DevSolveOp &op, const double *B, double *X, int nv
         a.prec = prec; a.plan = &pl; a.rpb = sh.rpb; a.sms = sm_count(); a.max_sms = max_sms;
         a.wait_limit = wait_limit > 0 ? wait_limit : SPIN_LIMIT;
         a.work = w + L.v; a.R = (double *)(w + L.r); a.part = (double *)(w + L.part);
-        a.bar = (unsigned *)(w + L.bar); a.err = (int *)(w + L.err); a.stats = stats_dev;
+        a.bar = (unsigned *)(w + L.bar); a.stats = stats_dev;
         return chs_solve(op, a, s);
     }
     if (!cheb && op.mgd && mgs_applicable(op)) {
         const Layout L = layout(op, nv, m, prec);
         char *w = (char *)work;
         cudaError_t e0;
-        if ((e0 = cudaMemsetAsync(w + L.bar, 0, L.total - L.bar, s)) != cudaSuccess) return e0;
+        if ((e0 = cudaMemsetAsync(w + L.bar, 0, L.ccnt - L.bar, s)) != cudaSuccess) return e0;
         if ((e0 = cudaMemsetAsync(stats_dev, 0, sizeof(GmresStats), s)) != cudaSuccess) return e0;
         MgsArgs a;
         a.B = B; a.X = X; a.nv = nv; a.ld = ld; a.m = m; a.max_iter = max_iter; a.tol = tol;
@@ -2635,7 +2630,7 @@ cudaError_t gmres_solve(const DevSolveOp &op, const double *B, double *X, int nv
         a.wait_limit = wait_limit > 0 ? wait_limit : SPIN_LIMIT;
         a.V = w + L.v; a.Z = w + L.z; a.Wv = w + L.w; a.R = (double *)(w + L.r);
         a.scratch = w + L.mg; a.part = (double *)(w + L.part);
-        a.bar = (unsigned *)(w + L.bar); a.err = (int *)(w + L.err); a.stats = stats_dev;
+        a.bar = (unsigned *)(w + L.bar); a.stats = stats_dev;
         return mgs_solve(op, a, s);
     }
     // cluster tail of the V-cycle: the levels [ncl, nred) in the group's first
@@ -2706,7 +2701,7 @@ cudaError_t gmres_solve(const DevSolveOp &op, const double *B, double *X, int nv
         memcpy(p.cheb_cb, pl.cb, sizeof pl.cb);
     }
     p.part = (double *)(w + L.part);
-    p.bar = (unsigned *)(w + L.bar); p.err = (int *)(w + L.err); p.stats = stats_dev;
+    p.bar = (unsigned *)(w + L.bar); p.err = &stats_dev->status; p.stats = stats_dev;
     p.groups = groups; p.G = G;
     p.wait_limit = wait_limit > 0 ? wait_limit : SPIN_LIMIT;
     p.cluster = CS;
@@ -2744,9 +2739,7 @@ cudaError_t gmres_solve(const DevSolveOp &op, const double *B, double *X, int nv
     cfg.numAttrs = CS > 0 ? 2 : 1;
     e = cudaLaunchKernelExC(&cfg, fn, args);
     if (e != cudaSuccess) return e;
-    g_kernel_launches += 2;
-    // a barrier timeout lands in stats->status (2)
-    fold_err<<<1, 1, 0, s>>>(p.err, stats_dev);
+    ++g_kernel_launches;
     if (p.timers) {   // debug: print block 0's phase cycles for this launch
         long long h[T_NPHASE];
         GmresStats st;
@@ -2767,7 +2760,7 @@ cudaError_t gmres_solve(const DevSolveOp &op, const double *B, double *X, int nv
 // Workspace of a multi-operator launch: the per-RHS vectors of every segment
 // back to back, one group scratch sized for the largest hierarchy.
 struct MultiLayout {
-    size_t v, z, w, r, mg, part, bar, err, ccnt, total;
+    size_t v, z, w, r, mg, part, bar, ccnt, total;
     size_t voff[MAXSEG], zoff[MAXSEG], woff[MAXSEG], roff[MAXSEG];
 };
 
@@ -2795,8 +2788,7 @@ static MultiLayout multi_layout(const DevSolveOp *const *ops, const int *nvk, in
     L.mg = L.r + al(8 * er);
     L.part = L.mg + al(es * ge * (size_t)groups);
     L.bar = L.part + al(8 * (size_t)4096 * 2 * (MAXM + 2));
-    L.err = L.bar + al(8 * (size_t)GROUPS_CAP);
-    L.ccnt = L.err + 256;
+    L.ccnt = L.bar + al(8 * (size_t)GROUPS_CAP);
     L.total = L.ccnt + al(8 * (size_t)GROUPS_CAP);
     return L;
 }
@@ -2879,7 +2871,7 @@ cudaError_t gmres_solve_multi(const DevSolveOp *const *ops, const int *nvk, cons
     p.cheb_k = 0;
     p.cheb_lg = p.cheb_ls = 0.0;
     p.part = (double *)(w + L.part);
-    p.bar = (unsigned *)(w + L.bar); p.err = (int *)(w + L.err); p.stats = stats_dev;
+    p.bar = (unsigned *)(w + L.bar); p.err = &stats_dev->status; p.stats = stats_dev;
     p.groups = groups; p.G = G;
     p.wait_limit = wait_limit > 0 ? wait_limit : SPIN_LIMIT;
     p.cluster = 0;
@@ -2923,8 +2915,7 @@ cudaError_t gmres_solve_multi(const DevSolveOp *const *ops, const int *nvk, cons
     cfg.attrs = coop;
     cfg.numAttrs = 1;
     if ((e = cudaLaunchKernelExC(&cfg, fn, args)) != cudaSuccess) return e;
-    g_kernel_launches += 2;
-    fold_err<<<1, 1, 0, s>>>(p.err, stats_dev);
+    ++g_kernel_launches;
     return cudaGetLastError();
 }
 

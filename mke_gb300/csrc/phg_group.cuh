@@ -6,6 +6,7 @@
 namespace phg {
 
 constexpr int MAXM = 48;         // largest restart length
+constexpr int STATUS_TIMEOUT = 2;  // GmresStats::status of a launch that gave up a wait (also its error flag)
 constexpr long long SPIN_LIMIT = 2000000000LL;  // default wait limit, clock64 cycles (~1 s)
 
 // phase cycle counters kept by block 0 when PHG_PHASE_TIMING is set
@@ -65,7 +66,7 @@ __device__ bool group_sync(unsigned *bar, int G, int *err, long long *tm) {
         while ((v = ld_relaxed(cnt)) < target) {   // the poison bit is above any target
             if (clock64() - t0 > lim) {
                 atomicOr(cnt, BAR_POISON);
-                atomicExch(err, 1);
+                atomicMax(err, STATUS_TIMEOUT);
                 v = BAR_POISON;
                 break;
             }

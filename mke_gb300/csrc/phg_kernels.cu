@@ -76,31 +76,43 @@ __global__ void k_apply(DevEll A, DevCols C, const double *xin, int ldx, const i
 // the 8 derivative right-hand sides of SphereJacobian::calc2
 // (src/sjacobian.cpp:136-362), out[(v * 8 + k) * ldo + i]:
 //   k: 0 D2c u, 1 D1 v, 2 D1c u, 3 D2 v, 4 D2 u, 5 D1c v, 6 D1 u, 7 D2c v
-__global__ void k_jac_rhs(JacOps J, const double *u, const double *w, int ld, const int *imap,
-                          const int *bmap, double *out, int ldo, int nv) {
-    const int n = J.d1.n;
-    const long long total = (long long)nv * n;
+// Bound by the FP64 pipe for many members (112 separate multiplies and adds per
+// row and member) and by latency for one: half a row per thread (the four
+// products of one field), all its gathers issued together (level 6, one
+// member: 25.4 -> 13.7 us).
+__global__ void __launch_bounds__(TB) k_jac_rhs(JacOps J, const double *u, const double *w, int ld, const int *imap,
+                                                const int *bmap, double *out, int ldo, int nv) {
+    const int n = J.d1.n, W = J.d1.W;
+    const long long total = 2LL * nv * n;
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
-        int v = (int)(t / n), i = (int)(t % n);
-        const double *fu = u + (size_t)v * ld, *fv = w + (size_t)v * ld;
-        double s[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-        for (int k = 0; k < J.d1.W; ++k) {
-            size_t e = (size_t)k * n + i;
-            int c = __ldg(&J.d1.col[e]);
-            int cc = imap ? imap[c] : c;
-            double xu = fu[cc], xv = fv[cc];
-            double a1 = __ldg(&J.d1.val[e]), a2 = __ldg(&J.d2.val[e]);
-            double c1 = __ldg(&J.d1c.val[e]), c2 = __ldg(&J.d2c.val[e]);
-            s[0] += c2 * xu; s[1] += a1 * xv; s[2] += c1 * xu; s[3] += a2 * xv;
-            s[4] += a2 * xu; s[5] += c1 * xv; s[6] += a1 * xu; s[7] += c2 * xv;
+        const int f = (int)(t / n), i = (int)(t - (long long)f * n), v = f >> 1;
+        const bool on_u = (f & 1) == 0;
+        const double *x = (on_u ? u : w) + (size_t)v * ld;
+        double s1 = 0.0, s2 = 0.0, c1 = 0.0, c2 = 0.0;   // D1, D2, D1cos, D2cos times the field
+        for (int k0 = 0; k0 < W; k0 += 8) {
+            double xv[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                if (k0 + k < W) {
+                    const int c = __ldg(&J.d1.col[(size_t)(k0 + k) * n + i]);
+                    xv[k] = x[imap ? imap[c] : c];
+                }
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                if (k0 + k < W) {
+                    const size_t e = (size_t)(k0 + k) * n + i;
+                    s1 += __ldg(&J.d1.val[e]) * xv[k]; s2 += __ldg(&J.d2.val[e]) * xv[k];
+                    c1 += __ldg(&J.d1c.val[e]) * xv[k]; c2 += __ldg(&J.d2c.val[e]) * xv[k];
+                }
         }
-        const double *bu = fu, *bv = fv;
-        double b[8];
-        b[0] = cols_sum(J.d2cb, bu, bmap, i); b[1] = cols_sum(J.d1b, bv, bmap, i);
-        b[2] = cols_sum(J.d1cb, bu, bmap, i); b[3] = cols_sum(J.d2b, bv, bmap, i);
-        b[4] = cols_sum(J.d2b, bu, bmap, i); b[5] = cols_sum(J.d1cb, bv, bmap, i);
-        b[6] = cols_sum(J.d1b, bu, bmap, i); b[7] = cols_sum(J.d2cb, bv, bmap, i);
-        for (int k = 0; k < 8; ++k) out[((size_t)v * 8 + k) * ldo + i] = b[k] + s[k];
+        const double b1 = cols_sum(J.d1b, x, bmap, i), b2 = cols_sum(J.d2b, x, bmap, i);
+        const double e1 = cols_sum(J.d1cb, x, bmap, i), e2 = cols_sum(J.d2cb, x, bmap, i);
+        double *o = out + (size_t)v * 8 * ldo + i;
+        if (on_u) {
+            o[0] = e2 + c2; o[2 * (size_t)ldo] = e1 + c1; o[4 * (size_t)ldo] = b2 + s2; o[6 * (size_t)ldo] = b1 + s1;
+        } else {
+            o[(size_t)ldo] = b1 + s1; o[3 * (size_t)ldo] = b2 + s2; o[5 * (size_t)ldo] = e1 + c1; o[7 * (size_t)ldo] = e2 + c2;
+        }
     }
 }
 
@@ -140,6 +152,25 @@ __global__ void k_p2u(double *u, int ldu, const double *p, int ldp, const double
     }
 }
 
+// k_p2u of an inner vector and the apply y = A p + C xb of the same vector in
+// one launch (a time step's solution, and the next solve's right-hand side)
+__global__ void k_p2u_apply(double *u, const double *p, const double *bnd, int ldb, const int *p2io, const int *isb,
+                            DevEll A, DevCols C, const double *xb, double *y, int V, int nv) {
+    const long long total = (long long)nv * V;
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)gridDim.x * blockDim.x) {
+        const int v = (int)(t / V), i = (int)(t % V), j = p2io[i];
+        if (isb[i]) {
+            u[t] = bnd ? bnd[(size_t)v * ldb + j] : 0.0;
+            continue;
+        }
+        const double *x = p + (size_t)v * A.n;
+        u[t] = x[j];
+        double s = row_sum(A, x, nullptr, j);
+        if (C.ptr && xb) s = s + cols_sum(C, xb + (size_t)v * ldb, nullptr, j);
+        y[(size_t)v * A.n + j] = s;
+    }
+}
+
 // y = a * x + b * z (both products rounded, then the sum) -- vec_sum1
 __global__ void k_axpbz(double *y, const double *x, double a, const double *z, double b, long long n) {
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x)
@@ -172,38 +203,56 @@ __global__ void k_bv_mix(double *tmp1, double *tmp2, const double *w_n, const do
     }
 }
 
-// elementwise a - b
-__global__ void k_sub(double *y, const double *a, const double *b, long long n) {
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x)
-        y[t] = a[t] - b[t];
-}
-
-// per-member partial sums of a[i] * b[i] over chunks of `chunk` rows
-__global__ void k_dot_partial(const double *a, const double *b, int ld, int n, int chunk, int nchunk,
-                              double *part, int nv) {
-    __shared__ double red[TB];
-    int v = blockIdx.x / nchunk, c = blockIdx.x % nchunk;
-    if (v >= nv) return;
-    const double *x = a + (size_t)v * ld, *y = b + (size_t)v * ld;
-    int i0 = c * chunk, i1 = min(n, i0 + chunk);
+// SphereNorm's products in one pass: per member the partial sums over chunks of
+// NORM_CHUNK rows of a_i (NORM b)_i, or, for a distance, of d_i (NORM d)_i with
+// d = a - b formed on the fly (one launch and no vector written, where the
+// difference, the product and the sum were three)
+constexpr int NORM_CHUNK = 1024;
+__global__ void __launch_bounds__(TB) k_norm_partial(DevEll A, const double *a, const double *b, int nchunk, int dist,
+                                                     double *part) {
+    __shared__ double red[TB / 32];
+    const int v = blockIdx.x / nchunk, c = blockIdx.x % nchunk, n = A.n;
+    const double *x = a + (size_t)v * n, *y = b + (size_t)v * n;
+    const int i1 = min(n, (c + 1) * NORM_CHUNK);
     double s = 0.0;
-    for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) s += x[i] * y[i];
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if (threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-        __syncthreads();
+    for (int i = c * NORM_CHUNK + threadIdx.x; i < i1; i += TB) {
+        if (dist) {
+            double r = 0.0;
+            for (int k0 = 0; k0 < A.W; k0 += 8) {
+                double d[8];
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+                    if (k0 + k < A.W) {
+                        const int q = __ldg(&A.col[(size_t)(k0 + k) * n + i]);
+                        d[k] = x[q] - y[q];
+                    }
+#pragma unroll
+                for (int k = 0; k < 8; ++k)
+                    if (k0 + k < A.W) r += __ldg(&A.val[(size_t)(k0 + k) * n + i]) * d[k];
+            }
+            s += (x[i] - y[i]) * r;
+        } else {
+            s += x[i] * row_sum(A, y, nullptr, i);
+        }
     }
-    if (threadIdx.x == 0) part[blockIdx.x] = red[0];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double t = 0.0;
+        for (int k = 0; k < TB / 32; ++k) t += red[k];
+        part[blockIdx.x] = t;
+    }
 }
 
-// out[v] = sum of the member's partials (sqrt if take_sqrt)
-__global__ void k_dot_final(const double *part, int nchunk, double *out, int nv, int take_sqrt) {
-    int v = blockIdx.x * blockDim.x + threadIdx.x;
+// out[v] = sum of the member's partials (sqrt if take_sqrt), one warp per member
+__global__ void __launch_bounds__(TB) k_norm_final(const double *part, int nchunk, double *out, int nv, int take_sqrt) {
+    const int v = blockIdx.x * (TB / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (v >= nv) return;
     double s = 0.0;
-    for (int c = 0; c < nchunk; ++c) s += part[(size_t)v * nchunk + c];
-    out[v] = take_sqrt ? sqrt(s) : s;
+    for (int c = lane; c < nchunk; c += 32) s += part[(size_t)v * nchunk + c];
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane == 0) out[v] = take_sqrt ? sqrt(s) : s;
 }
 
 // Picard bookkeeping: u_n <- u_n1 for members still iterating, then stop a
@@ -354,7 +403,7 @@ cudaError_t apply_op(const DevEll &A, const DevCols &C, const double *xin, int l
 
 cudaError_t jac_rhs(const JacOps &J, const double *u, const double *v, int ld, const int *imap,
                     const int *bmap, double *out, int ldo, int nv, cudaStream_t s) {
-    k_jac_rhs<<<grid_for((long long)nv * J.d1.n), TB, 0, s>>>(J, u, v, ld, imap, bmap, out, ldo, nv);
+    k_jac_rhs<<<grid_for(2LL * nv * J.d1.n), TB, 0, s>>>(J, u, v, ld, imap, bmap, out, ldo, nv);
     g_kernel_launches++;
     return cudaGetLastError();
 }
@@ -394,21 +443,21 @@ cudaError_t bv_mix(double *tmp1, double *tmp2, const double *w_n, const double *
     return cudaGetLastError();
 }
 
-cudaError_t vsub(double *y, const double *a, const double *b, long long n, cudaStream_t s) {
-    k_sub<<<grid_for(n), TB, 0, s>>>(y, a, b, n);
+cudaError_t p2u_apply(double *u, const double *p, const double *bnd, int ldb, const int *p2io, const int *isb, int V,
+                      const DevEll &A, const DevCols &C, const double *xb, double *y, int nv, cudaStream_t s) {
+    k_p2u_apply<<<grid_for((long long)nv * V), TB, 0, s>>>(u, p, bnd, ldb, p2io, isb, A, C, xb, y, V, nv);
     g_kernel_launches++;
     return cudaGetLastError();
 }
 
-int dot_chunks(int n) { return (n + 8191) / 8192; }
+int norm_chunks(int n) { return (n + NORM_CHUNK - 1) / NORM_CHUNK; }
 
-cudaError_t dot(const double *a, const double *b, int ld, int n, int nv, double *part, double *out,
-                bool take_sqrt, cudaStream_t s) {
-    int nch = dot_chunks(n);
-    k_dot_partial<<<nv * nch, TB, 0, s>>>(a, b, ld, n, 8192, nch, part, nv);
-    g_kernel_launches++;
-    k_dot_final<<<(nv + 127) / 128, 128, 0, s>>>(part, nch, out, nv, take_sqrt ? 1 : 0);
-    g_kernel_launches++;
+cudaError_t norm_dot(const DevEll &A, const double *a, const double *b, bool dist, int nv, double *part, double *out,
+                     bool take_sqrt, cudaStream_t s) {
+    const int nch = norm_chunks(A.n);
+    k_norm_partial<<<nv * nch, TB, 0, s>>>(A, a, b, nch, dist ? 1 : 0, part);
+    k_norm_final<<<(nv + TB / 32 - 1) / (TB / 32), TB, 0, s>>>(part, nch, out, nv, take_sqrt ? 1 : 0);
+    g_kernel_launches += 2;
     return cudaGetLastError();
 }
 

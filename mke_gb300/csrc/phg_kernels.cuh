@@ -34,11 +34,14 @@ cudaError_t bv_fc(double *FC, const double *w, const double *dw, const double *r
 cudaError_t bv_mix(double *tmp1, double *tmp2, const double *w_n, const double *w, const double *u_n,
                    const double *u, const double *lh, int V, double a1, double a2, double k2, double t1,
                    double t2, long long n, cudaStream_t s);
-cudaError_t vsub(double *y, const double *a, const double *b, long long n, cudaStream_t s);
-int dot_chunks(int n);
-// out[v] = sum_i a[v][i] b[v][i] (sqrt if take_sqrt); part holds nv * dot_chunks(n) doubles
-cudaError_t dot(const double *a, const double *b, int ld, int n, int nv, double *part, double *out,
-                bool take_sqrt, cudaStream_t s);
+// p2u of the inner vectors p (leading dimension A.n) into u, and y = A p + C xb
+cudaError_t p2u_apply(double *u, const double *p, const double *bnd, int ldb, const int *p2io, const int *isb, int V,
+                      const DevEll &A, const DevCols &C, const double *xb, double *y, int nv, cudaStream_t s);
+int norm_chunks(int n);
+// out[v] = sum_i a_i (A b)_i, or with d = a - b sum_i d_i (A d)_i (sqrt if
+// take_sqrt), vectors of A.n; part holds nv * norm_chunks(A.n) doubles
+cudaError_t norm_dot(const DevEll &A, const double *a, const double *b, bool dist, int nv, double *part, double *out,
+                     bool take_sqrt, cudaStream_t s);
 cudaError_t bv_commit(double *u_n, const double *u_n1, const double *nr, const double *nr0, int *done,
                       int V, int nv, cudaStream_t s);
 cudaError_t gather(double *y, int ldy, const double *x, int ldx, const int *map, int n, int nv, cudaStream_t s);

@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
     double *red = hcol + MAXM + 2;           // (MAXM + 2) x RS partial sums of the warps
     VT *hv = (VT *)(red + (MAXM + 2) * RS);  // the column in the Krylov precision
     __shared__ Rows<VT> tab[N_TAB];
-    __shared__ double scal[4], s_inv, s_a, s_target;
+    __shared__ double scal[5], s_inv, s_a, s_target;
     __shared__ int s_stop, s_dead;
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -356,16 +356,20 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
                 }
                 __syncthreads();
             }
-            if (threadIdx.x == 0) {
-                const double bt = sqrt(hcol[0]), bn = cycles == 0 ? sqrt(hcol[1]) : bnorm;
-                scal[0] = bn;
-                scal[1] = bt;
-                scal[2] = bn > 0.0 ? bt / bn : (bn == 0.0 ? 0.0 : bn);
-                scal[3] = bt > 0.0 ? 1.0 / bt : 0.0;
-                s_target = fmax(tol * bn, inner_rtol * bt);
-                g[0] = bt;
-#pragma unroll 1
-                for (int l = 1; l <= m; ++l) g[l] = 0.0;
+            if (threadIdx.x < 2) {   // ||r|| and, the first time, ||b|| with their reciprocals, side by side
+                const double q = hcol[threadIdx.x], ri = q > 0.0 ? rsqrt(q) : 0.0;
+                const double nrm = q > 0.0 ? q * ri : q;   // NaN stays NaN
+                if (threadIdx.x == 0) { scal[1] = nrm; scal[3] = ri; }
+                else if (cycles == 0) { scal[0] = nrm; scal[4] = ri; }
+                __syncwarp(3u);
+                if (threadIdx.x == 0) {
+                    const double bn = scal[0];
+                    scal[2] = bn > 0.0 ? nrm * scal[4] : (bn == 0.0 ? 0.0 : bn);
+                    s_target = fmax(tol * bn, inner_rtol * nrm);
+                    g[0] = nrm;
+                }
+            } else if (threadIdx.x >= 32 && threadIdx.x < 32 + m) {
+                g[threadIdx.x - 31] = 0.0;
             }
             __syncthreads();
             bnorm = scal[0];
@@ -537,7 +541,13 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
                     if (ONE) __syncthreads();
                 }
                 if (bot == 1 && !helper) apply_tb();
-                // dense: x_top = [T b +] E b_bot
+                // dense: x_top = [T b +] E b_bot (the first row's T b while b_bot is on its way)
+                VT tb0 = 0;
+                if (!helper && top > 0 && top < bot && warp < C * (d1 - d0)) {
+                    const Rows<VT> &A = tab[TAB_T + top];
+                    const size_t e = (size_t)(d0 + warp / C - A.base) * MGX_WT;
+                    tb0 = row_sum<VT, ONE, MGX_WT, 1, C>(A.c + e, A.v + e, cells + p.boff[top] + warp % C, ep, wt);
+                }
                 if (!helper) {
                     const E *src = bot == 0 ? c0 : cells + p.boff[bot];
 #pragma unroll 1
@@ -565,6 +575,8 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
                                 ST::get(t1, ct, ci, ep, wt);
                                 tb = t1[0];
                             }
+                        } else if (top < bot && t == warp) {
+                            tb = tb0;
                         } else if (top < bot) {   // level top = bot - 1
                             const Rows<VT> &A = tab[TAB_T + top];
                             const size_t e = (size_t)(i - A.base) * MGX_WT;
@@ -795,10 +807,6 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
     }
 }
 
-__global__ void mgs_fold_err(const int *err, GmresStats *st) {
-    if (*err) st->status = 2;
-}
-
 size_t mgs_fixed_smem() {
     return sizeof(double) * ((MAXM + 1) * MAXM + 2 * MAXM + (MAXM + 1) + MAXM + (MAXM + 2) + (MAXM + 2) * RS) +
            sizeof(double) * (MAXM + 2);
@@ -969,7 +977,7 @@ cudaError_t mgs_solve(const DevSolveOp &op, const MgsArgs &q, cudaStream_t s) {
     p.part = q.part;
     // the stamped sums behind the plain ones: 2 (MAXM + 2) doubles a block each
     p.cpart = (char *)(q.part + (size_t)groups * G * 2 * (MAXM + 2));
-    p.bar = q.bar; p.err = q.err; p.stats = q.stats;
+    p.bar = q.bar; p.err = &q.stats->status; p.stats = q.stats;
     p.groups = groups; p.G = G;
     p.wait_limit = q.wait_limit;
     size_t c = (blk ? 8 : 2) * (size_t)n;
@@ -1001,8 +1009,7 @@ cudaError_t mgs_solve(const DevSolveOp &op, const MgsArgs &q, cudaStream_t s) {
     cfg.numAttrs = 1;
     void *args[] = {&p};
     if ((e = cudaLaunchKernelExC(&cfg, mgs_fn(q.prec, blk ? 2 : one ? 1 : 0), args)) != cudaSuccess) return e;
-    mgs_fold_err<<<1, 1, 0, s>>>(q.err, q.stats);
-    g_kernel_launches += 2;
+    ++g_kernel_launches;
     return cudaGetLastError();
 }
 

@@ -17,9 +17,8 @@ struct MgsArgs {
     double *R;             // nv x n
     void *scratch;         // min(nv, GROUPS_CAP) x mgs_scratch_bytes
     double *part;          // partial sums of the blocks
-    unsigned *bar;         // zeroed with err before the launch
-    int *err;
-    GmresStats *stats;     // zeroed before the launch
+    unsigned *bar;         // zeroed before the launch
+    GmresStats *stats;     // zeroed before the launch; its status is the launch's error flag
 };
 
 bool mgs_applicable(const DevSolveOp &op);

@@ -58,7 +58,7 @@ __device__ __forceinline__ void ld_cell(const ulonglong2 *p, double &v, unsigned
 
 // what a waiting warp needs to give up
 struct Waits {
-    int *err;                   // the launch's error flag
+    int *err;                   // the launch's error flag (the status of its record)
     unsigned long long *bar;    // the group's barrier word
     int *dead;                  // shared: this block gives up
     unsigned rounds;            // loads a wait may repeat: the wait limit at about 400 cycles (a trip to L2) each
@@ -82,9 +82,9 @@ __device__ __forceinline__ void wait_cells(VT (&x)[N], const Cell<VT> *p, const 
         if (!__any_sync(0xffffffffu, miss != 0)) return;
         if ((round & 63u) == 63u) {   // inline: a call here would put a register save at every wait
             const bool late = round >= w.rounds;
-            if (__any_sync(0xffffffffu, late || *(volatile int *)w.dead || *(volatile int *)w.err)) {
+            if (__any_sync(0xffffffffu, late || *(volatile int *)w.dead || *(volatile int *)w.err == STATUS_TIMEOUT)) {
                 if (late) {
-                    atomicExch(w.err, 1);
+                    atomicMax(w.err, STATUS_TIMEOUT);
                     atomicOr(w.bar, BAR_POISON);
                 }
                 *(volatile int *)w.dead = 1;
