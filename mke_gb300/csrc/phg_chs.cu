@@ -107,9 +107,10 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 1024 : 768, 1) chs_kernel(co
     }
     const VT c0 = (VT)p.c0;
     unsigned ep = 0;           // stamp of the last iterate written
-    int my_iters = 0, my_cycles = 0, my_status = 0, my_steps = 0;   // thread 0's
-    double my_rel = 0.0, my_bytes = 0.0;
-    const double es = (double)sizeof(VT), nrows = (double)cnt;
+    // (FP64 scalars are one thread's business: the FP64 pipe takes 16 cycles per
+    // warp instruction)
+    int my_iters = 0, my_cycles = 0, my_status = 0, my_steps = 0, my_rsteps = 0, my_resid = 0, my_upd = 0;
+    double my_rel = 0.0;
 
     for (int ch = grp; ch * C < nv; ch += p.groups) {
         const int v0 = ch * C, nc = min(C, nv - v0);
@@ -234,7 +235,7 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 1024 : 768, 1) chs_kernel(co
                 if (lane == 0) s_kc = kc;
             }
             __syncthreads();
-            my_bytes += nrows * (W * 12.0 + 24.0 * nc);
+            ++my_resid;
             if (first) {   // zero right-hand sides: x = 0
 #pragma unroll 1
                 for (int v = 0; v < nc; ++v)
@@ -247,11 +248,11 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 1024 : 768, 1) chs_kernel(co
             // e_1 = d_0 = c0 D^-1 r; r holds D^-1 r / ||r|| (zero for closed members)
 #pragma unroll 1
             for (int i = threadIdx.x; i < cnt; i += NT) {
-                const double di = __ldg(&p.dinv[r0 + i]);
+                const VT di = (VT)__ldg(&p.dinv[r0 + i]);
 #pragma unroll
                 for (int v = 0; v < C; ++v) {
                     VT q = 0;
-                    if (v < nc && s_open[v]) q = (VT)(p.R[(size_t)(v0 + v) * n + r0 + i] * s_scale[v] * di);
+                    if (v < nc && s_open[v]) q = (VT)(p.R[(size_t)(v0 + v) * n + r0 + i] * s_scale[v]) * di;
                     r[i * C + v] = q;
                     d[i * C + v] = c0 * q;
                     ST::put(e0 + (size_t)(r0 + i) * C + v, c0 * q, ep + 1);
@@ -287,7 +288,8 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 1024 : 768, 1) chs_kernel(co
                 E *t = ec; ec = en; en = t;
             }
             for (int v = 0; v < nc; ++v) my_steps += s_open[v] ? Kc - 1 : 0;
-            my_bytes += (Kc - 1) * nrows * (7 * (4.0 + es) + 7.0 * es * nc) + nrows * nc * (es + 16.0);
+            my_rsteps += Kc - 1;
+            ++my_upd;
             if (__syncthreads_or(s_dead)) return;
             // x += ||r|| e
 #pragma unroll 1
@@ -310,7 +312,11 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 1024 : 768, 1) chs_kernel(co
         // the next chunk reuses the cells
         if ((ch + p.groups) * C < nv && !group_sync(bar, G, err, nullptr)) return;
     }
-    if (threadIdx.x == 0) atomicAdd(&p.stats->bytes, my_bytes);
+    if (threadIdx.x == 0) {   // algorithmic bytes: residuals, steps (rows once for the chunk), updates
+        const double es = (double)sizeof(VT), c = min(C, nv);
+        atomicAdd(&p.stats->bytes, (double)cnt * (my_resid * (W * 12.0 + 24.0 * c) + my_rsteps * 7.0 * (4.0 + es) +
+                                                  my_steps * 7.0 * es + my_upd * c * (es + 16.0)));
+    }
     if (threadIdx.x == 0 && bi == 0) {
         atomicAdd(&p.stats->steps_total, my_steps);
         atomicMax(&p.stats->iters, my_iters);

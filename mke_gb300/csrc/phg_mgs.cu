@@ -93,7 +93,7 @@ struct MgsParams {
     int ncopy;
     const void *dense, *dense2;
     int off_d, off_d2;         // the dense rows in shared memory (-1: in global memory)
-    int off_w, off_v;          // own rows of A z (-1: in Wv) and of the Krylov vectors
+    int off_w, off_t, off_v;   // own rows of A z (-1: in Wv), of T b (-1: not kept), of the Krylov vectors
     int mv, mvp;               // Krylov vectors kept in shared memory, and the rows there are for them
     int off_b;                 // the dense product's input
 };
@@ -114,16 +114,19 @@ __device__ __forceinline__ VT row_sum(const int *col, const VT *v, const typenam
 #pragma unroll
     for (int q = 0; q < N; ++q) c[q] = C * col[KS * q];
     CellStore<VT, ONE>::get(x, p, c, stamp, w);
-    VT s = 0;
+    VT s = 0, t = 0;   // two chains: a dependent FP64 multiply-add takes 81 cycles
 #pragma unroll
-    for (int q = 0; q < N; ++q) s += v[KS * q] * x[q];
-    return s;
+    for (int q = 0; q < N; ++q) {
+        if (sizeof(VT) == 8 && (q & 1)) t += v[KS * q] * x[q];
+        else s += v[KS * q] * x[q];
+    }
+    return sizeof(VT) == 8 ? s + t : s;
 }
 
 // a dense row (16-byte aligned, length a multiple of four) times b, in every lane
 template <typename VT>
 __device__ __forceinline__ VT dense_row(const VT *row, const VT *b, int len, int lane) {
-    VT s = 0, s1 = 0;
+    VT s = 0, s1 = 0, s2 = 0, s3 = 0;
     if constexpr (sizeof(VT) == 4) {
 #pragma unroll 3
         for (int k = lane; k < len / 4; k += 32) {
@@ -131,13 +134,17 @@ __device__ __forceinline__ VT dense_row(const VT *row, const VT *b, int len, int
             s += a.x * x.x; s1 += a.y * x.y; s += a.z * x.z; s1 += a.w * x.w;
         }
     } else {
-#pragma unroll 4
-        for (int k = lane; k < len / 2; k += 32) {
+#pragma unroll 2
+        for (int k = lane; k < len / 2; k += 64) {
             const double2 a = ((const double2 *)row)[k], x = ((const double2 *)b)[k];
             s += a.x * x.x; s1 += a.y * x.y;
+            if (k + 32 < len / 2) {
+                const double2 c = ((const double2 *)row)[k + 32], z = ((const double2 *)b)[k + 32];
+                s2 += c.x * z.x; s3 += c.y * z.y;
+            }
         }
     }
-    return warp_sum(s + s1);
+    return warp_sum((s + s1) + (s2 + s3));
 }
 
 // Sums over the group's blocks, the same bits in every block.  Each block
@@ -176,10 +183,12 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
     double *cs = H + (MAXM + 1) * MAXM, *sn = cs + MAXM, *g = sn + MAXM, *y = g + MAXM + 1;
     double *hcol = y + MAXM;                 // the current column
     double *red = hcol + MAXM + 2;           // (MAXM + 2) x RS partial sums of the warps
+    VT *redv = (VT *)red;                    // the same in the Krylov precision
     VT *hv = (VT *)(red + (MAXM + 2) * RS);  // the column in the Krylov precision
     __shared__ Rows<VT> tab[N_TAB];
-    __shared__ double scal[5], s_inv, s_a, s_target;
-    __shared__ int s_stop, s_dead;
+    __shared__ double scal[5], s_a, s_target;
+    __shared__ VT s_inv;
+    __shared__ int s_stop, s_dead, s_go, s_zero;
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int NW = (blockDim.x >> 5) - 1;    // worker warps; the last warp is the helper
@@ -286,9 +295,12 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
     asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
 
-    int my_iters = 0, my_cycles = 0, my_status = 0, my_steps = 0;
-    double my_rel = 0.0, my_bytes = 0.0;
-    const double nrows = (double)kn;
+    // Scalars in FP64 are one thread's business: the FP64 pipe takes 16 cycles
+    // per warp instruction, so a sum kept or a test made by all 25 warps costs as
+    // much as a hand-over.  Thread 0 decides a cycle's start (s_go); the byte
+    // count is formed from counters at the end.
+    int my_iters = 0, my_cycles = 0, my_status = 0, my_steps = 0, my_resid = 0, my_cols = 0;
+    double my_rel = 0.0;
     unsigned ep = 0;           // stamp of the current V-cycle
 
 #pragma unroll 1
@@ -297,11 +309,12 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
         double *x = p.X + (size_t)v * ld;
         VT *V = Vp + (size_t)v * (m + 1) * nk, *Z = Zp + (size_t)v * m * nk;
         VT *wl = p.off_w >= 0 ? (VT *)(smem + p.off_w) : (VT *)p.Wv + (size_t)v * nk + k0;   // own rows of A z
+        VT *tl = p.off_t >= 0 ? (VT *)(smem + p.off_t) : nullptr;   // own rows of T b (null: read from ct)
         double *R = p.R + (size_t)v * nk;
         // own rows of Krylov vector l
         auto vrow = [&](int l) -> VT * { return l < p.mv ? vsm + (size_t)l * rpb : V + (size_t)l * nk + k0; };
-        int iters = 0, cycles = 0, status = 1;
-        double beta_prev = 0.0, rel = 0.0, bnorm = 0.0;
+        int iters = 0, cycles = 0;
+        double beta_prev = 0.0;   // thread 0's
 #pragma unroll 1
         for (;;) {
             // r = b - A x (FP64, exact operator) and its norm; with ||b|| the first time
@@ -331,7 +344,7 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
                         const double bv = b[i], q = bv - t;
                         R[i] = q;
                         sr += q * q;
-                        sb += bv * bv;
+                        if (cycles == 0) sb += bv * bv;
                     }
                 if (warp < NA) {
                     sr = warp_sum(sr);
@@ -364,28 +377,29 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
                 __syncwarp(3u);
                 if (threadIdx.x == 0) {
                     const double bn = scal[0];
-                    scal[2] = bn > 0.0 ? nrm * scal[4] : (bn == 0.0 ? 0.0 : bn);
+                    const double rel = bn > 0.0 ? nrm * scal[4] : (bn == 0.0 ? 0.0 : bn);
                     s_target = fmax(tol * bn, inner_rtol * nrm);
                     g[0] = nrm;
+                    int go = 1, status = 0;
+                    if (rel <= tol) go = 0;   // also a zero right-hand side
+                    else if (iters >= max_iter || (cycles > 0 && !(nrm < 0.9999 * beta_prev))) { go = 0; status = 1; }
+                    beta_prev = nrm;
+                    s_go = go;
+                    s_zero = bn == 0.0;
+                    if (!go) {
+                        my_rel = max_nan(my_rel, rel);
+                        my_status = max(my_status, status);
+                    }
                 }
             } else if (threadIdx.x >= 32 && threadIdx.x < 32 + m) {
                 g[threadIdx.x - 31] = 0.0;
             }
             __syncthreads();
-            bnorm = scal[0];
-            const double beta = scal[1];
-            if (bnorm == 0.0) {
+            ++my_resid;
+            if (s_zero)
 #pragma unroll 1
                 for (int i = k0 + threadIdx.x; i < k0 + kn; i += blockDim.x) x[i] = 0.0;
-                status = 0; rel = 0.0;
-                break;
-            }
-            my_bytes += nrows * p.resid_row_bytes;
-            rel = scal[2];
-            if (rel <= tol) { status = 0; break; }
-            if (iters >= max_iter) { status = 1; break; }
-            if (cycles > 0 && !(beta < 0.9999 * beta_prev)) { status = 1; break; }
-            beta_prev = beta;
+            if (!s_go) break;
             ++cycles;
             if (!helper) {
                 const double ib = scal[3];
@@ -407,7 +421,7 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
                     // norm of the last step's vector, its rotation and the stopping test
                     if (j > 0) {
                         if (!ONE) asm volatile("bar.sync 1, %0;" ::"r"((int)blockDim.x) : "memory");
-                        double s = lane < NA ? red[lane] : 0.0;
+                        double s = lane < NA ? (double)redv[lane] : 0.0;
                         s = lanes_sum(s, NA);
                         VT q = (VT)s;
                         if constexpr (!ONE) {
@@ -435,11 +449,11 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
                             H[k * MAXM + k] = r;
                             g[k + 1] = -sn[k] * g[k];
                             g[k] = cs[k] * g[k];
-                            s_inv = ri;
+                            s_inv = (VT)ri;
                             s_stop = fabs(g[k + 1]) <= s_target || hn == 0.0 || j == m || iters + j >= max_iter;
                         }
                     } else if (lane == 0) {
-                        s_inv = 1.0;
+                        s_inv = (VT)1;
                         s_stop = 0;
                     }
                 }
@@ -533,7 +547,10 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
                                 const Rows<VT> &A = tab[TAB_T];
                                 const size_t e = (size_t)(min(i, r1 - 1) - A.base) * MGX_WT;
                                 const VT s = row_sum<VT, ONE, MGX_WT, 1, C>(A.c + e, A.v + e, c0 + q, ep, wt);
-                                if (i < r1) ST::put(ct + (size_t)C * i + q, s, ep);
+                                if (i < r1) {
+                                    ST::put(ct + (size_t)C * i + q, s, ep);
+                                    if (tl) tl[it] = s;
+                                }
                             }
                         }
                         if (l == 1) apply_tb();
@@ -558,23 +575,15 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
                         if (q < C * nb) bsm[(q % C) * nbs + q / C] = t[0];
                     }
                 }
-                if (__syncthreads_or(s_dead)) return;
-                jl = j;
-                if (s_stop) break;
-                const VT inv = (VT)s_inv;
-                if (!helper)
+                if (!helper) {
+                    asm volatile("bar.sync 2, %0;" ::"r"(NW * 32) : "memory");   // the workers: bsm complete
 #pragma unroll 1
                     for (int t = warp; t < C * (d1 - d0); t += NW) {
                         const int i = d0 + t / C, h = t % C;
                         const VT *row = dn + (size_t)(i - d0) * nbs;
                         VT tb = 0;   // [T b] of the row
                         if (top == 0) {
-                            if (bot > 0) {   // this block's own T b
-                                const int ci[1] = {i};
-                                VT t1[1];
-                                ST::get(t1, ct, ci, ep, wt);
-                                tb = t1[0];
-                            }
+                            if (bot > 0) tb = tl[i - r0];
                         } else if (top < bot && t == warp) {
                             tb = tb0;
                         } else if (top < bot) {   // level top = bot - 1
@@ -589,13 +598,12 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
                         }
                         VT s2 = dense_row<VT>(dn2 + (size_t)(i - d0) * nbs, bsm, nbs, lane);
                         if (lane == 0) {
-                            if (bot > 0) s2 += wl[i - r0];
-                            Z[(size_t)j * nk + i] = s * inv;
-                            wl[i - r0] = s2 * inv;
-                            vrow(j)[i - r0] *= inv;
+                            tl[i - r0] = s;   // z and A z, not normalised yet
+                            wl[i - r0] = bot > 0 ? s2 + wl[i - r0] : s2;
                         }
                     }
-                if (ONE || top == 0) __syncthreads();
+                }
+                if (ONE) __syncthreads();
                 // up: x_l = T b_l + U x_{l+1}
 #pragma unroll 1
                 for (int l = top - 1; l >= 1; --l) {
@@ -614,19 +622,35 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
                     }
                     if (ONE) __syncthreads();
                 }
+                // the helper's results: the stopping test and 1 / norm
+                if (__syncthreads_or(s_dead)) return;
+                jl = j;
+                if (s_stop) break;
+                const VT inv = s_inv;
                 // finest level: z = T b + U x_1 and A z = A T b + A U x_1, normalised
+                if (!BLK && top == 0 && !helper)
+#pragma unroll 1
+                    for (int q = threadIdx.x; q < kn; q += NW * 32) {
+                        Z[(size_t)j * nk + k0 + q] = tl[q] * inv;
+                        wl[q] *= inv;
+                        vrow(j)[q] *= inv;
+                    }
                 if ((BLK || top > 0) && !helper)
 #pragma unroll 1
                     for (int t = warp; t < tr; t += NW) {
                         const int it = t * 32 + lane, i = r0 + it / C, h = it % C, row = min(i, r1 - 1);
                         const Rows<VT> &F = tab[TAB_F];
                         const size_t e = (size_t)(row - F.base) * MGX_SF;
-                        const int ci[1] = {C * row + h};
                         int c[MGX_WF];
                         VT tb[1], x1[MGX_WF];
 #pragma unroll
                         for (int q = 0; q < MGX_WF; ++q) c[q] = C * (F.c + e)[q] + h;
-                        ST::get(tb, ct, ci, ep, wt);   // this block's own T b
+                        if (tl) {
+                            tb[0] = tl[min(it, C * (r1 - r0) - 1)];
+                        } else {   // this block's own T b
+                            const int ci[1] = {C * row + h};
+                            ST::get(tb, ct, ci, ep, wt);
+                        }
                         ST::get(x1, cells + p.xoff[1], c, ep, wt);
                         VT s = 0, aw = 0, ew = 0;
 #pragma unroll
@@ -653,7 +677,7 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
                         }
                     }
                 if (BLK) __syncthreads();   // the vectors' entries change hands
-                my_bytes += nrows * (p.step_row_bytes + es * 2.0 * (j + 1));
+                my_cols += j + 1;
                 // dots with v_0..v_j, eight basis vectors per pass, on this thread's own rows
                 if (warp < NA)
 #pragma unroll 1
@@ -681,12 +705,12 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
                         }
                         const VT s = fold8(t, lane);
                         const int k = lane >> 2;   // bits 4, 3, 2 of the lane: value 4 h16 + 2 h8 + h4
-                        if ((lane & 3) == 0 && k < kk) red[(l0 + k) * RS + warp] = (double)s;
+                        if ((lane & 3) == 0 && k < kk) redv[(l0 + k) * RS + warp] = s;
                     }
                 __syncthreads();
 #pragma unroll 1
                 for (int l = warp; l <= j; l += NW + 1) {
-                    double s = lane < NA ? red[l * RS + lane] : 0.0;
+                    double s = lane < NA ? (double)redv[l * RS + lane] : 0.0;
                     s = lanes_sum(s, NA);
                     const VT q = (VT)s;
                     if constexpr (ONE) {
@@ -750,7 +774,7 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
                     }
                     if (warp < NA) {
                         a2 = warp_sum(a2);
-                        if (lane == 0) red[warp] = (double)a2;
+                        if (lane == 0) redv[warp] = a2;
                     }
                     if (!ONE) asm volatile("bar.arrive 1, %0;" ::"r"((int)blockDim.x) : "memory");
                 }
@@ -786,17 +810,16 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
                     for (int l = 0; l < jl; ++l) s += hv[l] * Z[(size_t)l * nk + i];
                     x[i] += (double)s;
                 }
-            my_bytes += nrows * (jl * es + 24.0);
             if (!group_sync(bar, G, err, nullptr)) return;   // x complete
         }
         my_iters = max(my_iters, iters);
         my_cycles = max(my_cycles, cycles);
-        my_rel = max_nan(my_rel, rel);
-        my_status = max(my_status, status);
         // the next right-hand side reuses the cells and the shared memory
         if (v + p.groups < p.nv && !group_sync(bar, G, err, nullptr)) return;
     }
-    if (threadIdx.x == 0) atomicAdd(&p.stats->bytes, my_bytes);
+    if (threadIdx.x == 0)
+        atomicAdd(&p.stats->bytes, (double)kn * (my_resid * p.resid_row_bytes + my_steps * (p.step_row_bytes + es) +
+                                                 2.0 * es * my_cols + 24.0 * my_cycles));
     if (threadIdx.x == 0 && bi == 0) {
         atomicAdd(&p.stats->steps_total, my_steps);
         atomicMax(&p.stats->iters, my_iters);
@@ -915,6 +938,7 @@ cudaError_t mgs_solve(const DevSolveOp &op, const MgsArgs &q, cudaStream_t s) {
     p.off_b = take(C * es * (size_t)mgx_stride(x.lev[p.bot].n));
     if (p.off_b < 0) return cudaErrorInvalidValue;
     p.off_w = take(NK * es * rpb(0));
+    p.off_t = take(C * es * rpb(0));
     auto copy = [&](const void *src, int rows, int words, int dst) {
         Copy &c = p.copy[p.ncopy++];
         c.src = src; c.rows = rows; c.words = words; c.dst = dst;
