@@ -1438,7 +1438,7 @@ extern "C" int phg_ops_mult32(phg_ops o, const char *name, float *y, const float
     if (!v32) return fail(PHG_ERR_ARG, "no FP32 copy of '%s'", name);
     // row records where the operator has them (one matrix stream: 72 % of the HBM copy peak at level 8 x 64
     // vs 62 % for the slot-major arrays' 14 streams); the same bits either way
-    if (pk) CK(spmm_pk32(pk, o->rs, x, y, nv, o->str(stream)));
+    if (pk) CK(spmm_pk32(pk, o->rs, o->W, x, y, nv, o->str(stream)));
     else CK(spmm_il32(o->pcol.as<int>(), v32, o->rs, o->W, x, y, nv, o->str(stream)));
     return PHG_OK;
     PHG_API_END
@@ -1633,11 +1633,12 @@ int tune_spmm(phg_ops_s *o, int nv, cudaStream_t s, Report &rep) {
     CK(fill_hash32(x.as<float>(), (long long)len, 777u, s));
     float best = 1e30f;
     int pick = 0;
-    for (int tpr = 1; tpr <= q4; tpr *= 2) {
-        if (q4 / tpr > 8) continue;
+    const bool ruled = pk && spmm_walks(o->rs, o->W, nv);   // -1: the walking kernel, whatever the table says
+    for (int tpr = ruled ? -1 : 1; tpr <= q4; tpr = tpr < 0 ? 1 : 2 * tpr) {
+        if (tpr > 0 && q4 / tpr > 8) continue;
         float ms = 0.f;
         int r = time_best(s, 5, [&]() -> int {
-            if (pk) CK(spmm_pk32(pk, o->rs, x.as<float>(), y.as<float>(), nv, s, tpr));
+            if (pk) CK(spmm_pk32(pk, o->rs, o->W, x.as<float>(), y.as<float>(), nv, s, tpr));
             else CK(spmm_il32(o->pcol.as<int>(), v32, o->rs, o->W, x.as<float>(), y.as<float>(), nv, s, tpr));
             return PHG_OK;
         }, &ms);
@@ -1646,7 +1647,7 @@ int tune_spmm(phg_ops_s *o, int nv, cudaStream_t s, Report &rep) {
         if (ms < best) { best = ms; pick = tpr; }
     }
     if (pick) {
-        tune_set_spmm(o->rs, nv, pick);
+        tune_set_spmm(o->rs, nv, std::max(pick, 0));
         rep.add("chose spmm nv=%d threads_per_row=%d\n", nv, pick);
     }
     return PHG_OK;

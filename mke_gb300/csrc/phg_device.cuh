@@ -178,7 +178,8 @@ int solve_family(const DevSolveOp &op);
 bool tune_get_solve(int family, int n, Precision p, int nv, SolveShape *out);
 void tune_set_solve(int family, int n, Precision p, int nv, const SolveShape &s);
 bool tune_get_spmm(int n, int nv, int *tpr);
-void tune_set_spmm(int n, int nv, int tpr);
+void tune_set_spmm(int n, int nv, int tpr);   // 0: drop the entry
+int sm_count();   // the device's SMs
 void tune_clear();
 std::string tune_describe();
 int tune_save(const char *path);

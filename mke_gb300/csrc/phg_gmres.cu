@@ -1228,8 +1228,6 @@ size_t block_group_elems(const DevSolveOp &op) {
     return 2 * op.mg.group_elems + 4 * (size_t)(op.A.n / 4);
 }
 
-int sm_count();
-
 // whether gmres_solve runs op's solves as Chebyshev iterations (the same test)
 bool uses_cheb(const DevSolveOp &op, int m) {
     return op.cheb_lmax > 0.0 && op.cheb_lmin > 0.0 && op.cheb_lmin < op.cheb_lmax && m >= 3 && !op.mgd &&
@@ -1671,6 +1669,8 @@ cudaError_t cheb_lockstep(const DevSolveOp &op, const double *B, double *X, int 
 // the device's SM count, read once (serving lanes call this from several threads)
 std::atomic<int> g_sms{0};
 
+}  // namespace
+
 int sm_count() {
     int n = g_sms.load(std::memory_order_relaxed);
     if (!n) {
@@ -1681,6 +1681,8 @@ int sm_count() {
     }
     return n;
 }
+
+namespace {
 
 int env_int(const char *name, int dflt) {
     const char *e = getenv(name);

@@ -845,6 +845,66 @@ __global__ void __launch_bounds__(TB) k_spmm_pk(const uint4 *__restrict__ pk, in
     }
 }
 
+// Y = A X as k_spmm_pk, for long rows: a block owns one 128-byte slice (32
+// members) of a contiguous range of rows and walks it, 128 rows at a time.
+// The sphere's points are numbered along rings, so a row's neighbours lie at
+// most a ring away on either side, and the two rings of a slice (level 7:
+// 1,284 rows of 128 bytes, 164 KB) stay in the SM's L1, where scattered
+// blocks fetch each row of X from L2 three times over.  Level 7 x 128 members,
+// 178 MB at the least: 45.2 us scattered, 39.0 here (41.3 with buffers that
+// are not in L2), 4.3 TB/s.  What bounds it is the gathers' latency and their
+// way through the L1 (75 % of its cycles): with 24 warps 48 us, with 16 warps
+// 55.  So a block has 1,024 threads, the next row's record is loaded behind
+// this row's gathers, and the test for infinities costs one FMA per row (a
+// branch on it in the loop: 48 us).  Also measured: a window of rows in
+// shared memory filled by asynchronous copies 45, prefetches into L2 no gain,
+// a record shared by shuffles 42.
+// Seven gathers: the record's eighth slot is padding (host check).
+__global__ void __launch_bounds__(1024, 1) k_spmm_walk(const uint4 *__restrict__ pk, int n, int per,
+                                                       const float4 *__restrict__ x, float4 *__restrict__ y, int q4,
+                                                       int slices) {
+    const int range = blockIdx.x / slices, q = blockIdx.x % slices * 8 + (threadIdx.x & 7);
+    const int first = range * per + (int)(threadIdx.x >> 3), end = min(n, (range + 1) * per);
+    if (first >= end) return;
+    x += q; y += q;
+    uint4 e[4];   // the next row's record, without its padding
+    auto load = [&](int i) {
+#pragma unroll
+        for (int k = 0; k < 3; ++k) e[k] = __ldg(&pk[(size_t)i * 4 + k]);
+        const uint2 h = __ldg((const uint2 *)&pk[(size_t)i * 4 + 3]);
+        e[3] = make_uint4(h.x, h.y, 0, 0);
+    };
+    load(first);
+    float odd = 0.f;   // NaN once a sum was infinite or NaN
+    for (int i = first; i < end; i += 128) {
+        float a[7];
+        float4 g[7];
+#pragma unroll
+        for (int k = 0; k < 7; ++k) {   // n q4 < 2^31 (host check)
+            g[k] = __ldg(&x[((k & 1) ? e[k / 2].z : e[k / 2].x) * (unsigned)q4]);
+            a[k] = __uint_as_float((k & 1) ? e[k / 2].w : e[k / 2].y);
+        }
+        load(min(i + 128, end - 1));
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int k = 0; k < 7; ++k) {
+            s.x = __fmaf_rn(a[k], g[k].x, s.x); s.y = __fmaf_rn(a[k], g[k].y, s.y);
+            s.z = __fmaf_rn(a[k], g[k].z, s.z); s.w = __fmaf_rn(a[k], g[k].w, s.w);
+        }
+        odd = __fmaf_rn(0.f, (s.x + s.y) + (s.z + s.w), odd);
+        __stcs(&y[(unsigned)i * (unsigned)q4], s);
+    }
+    if (odd == 0.f) return;
+    // the padding's term, 0 x_i, which is NaN where x_i is infinite
+    for (int i = first; i < end; i += 128) {
+        const float4 d = __ldg(&x[(unsigned)i * (unsigned)q4]);
+        float4 s = y[(unsigned)i * (unsigned)q4];
+        s.x = __fmaf_rn(0.f, d.x, s.x); s.y = __fmaf_rn(0.f, d.y, s.y);
+        s.z = __fmaf_rn(0.f, d.z, s.z); s.w = __fmaf_rn(0.f, d.w, s.w);
+        y[(unsigned)i * (unsigned)q4] = s;
+    }
+}
+
 }  // namespace
 
 template <typename T>
@@ -861,11 +921,31 @@ template cudaError_t spmm<double>(const int *, const double *, int, int, const d
 template cudaError_t spmm<float>(const int *, const float *, int, int, const float *, int, float *, int, int,
                                  cudaStream_t);
 
-cudaError_t spmm_pk32(const unsigned *pk, int n, const float *x, float *y, int nv, cudaStream_t s, int tpr) {
+// Where the walk is the faster one (us, walk / scattered, buffers not in L2):
+// level 7 x 256 77 / 92, x 128 41 / 45, level 6 x 256 22 / 31, x 128 13.6 /
+// 16.5, x 32 6.3 / 7.2, level 5 x 128 7.0 / 8.3, level 4 x 256 6.3 / 12; but
+// level 5 x 64, in L2, 6.1 / 5.2: too few rows per block.  Above 2^18 rows
+// (level 8) two rings of a slice no longer fit the L1: x 64 92 / 76, x 128
+// 174 / 152, and only x 256 gains, 330 / 364.
+bool spmm_walks(int n, int W, int nv) {
+    return W <= 7 && nv % 32 == 0 && (long long)n * nv < (1LL << 33) &&
+           (nv >= 128 || (long long)n * nv >= (1LL << 20)) && (n <= (1 << 18) || nv >= 256);
+}
+
+cudaError_t spmm_pk32(const unsigned *pk, int n, int W, const float *x, float *y, int nv, cudaStream_t s, int tpr) {
     if (n < 1 || nv < 4 || nv % 4 || ((uintptr_t)x & 15) || ((uintptr_t)y & 15) || ((uintptr_t)pk & 15))
         return cudaErrorInvalidValue;
     const int q4 = nv / 4;
-    if (tpr <= 0) tune_get_spmm(n, nv, &tpr);
+    const uint4 *p4 = (const uint4 *)pk;
+    if (tpr == 0) tune_get_spmm(n, nv, &tpr);
+    if (tpr <= 0 && spmm_walks(n, W, nv)) {
+        const int slices = q4 / 8, ranges = std::max(1, sm_count() / slices);
+        const int per = (n + ranges - 1) / ranges;
+        k_spmm_walk<<<(unsigned)(ranges * slices), 1024, 0, s>>>(p4, n, per, (const float4 *)x, (float4 *)y, q4,
+                                                                slices);
+        g_kernel_launches++;
+        return cudaGetLastError();
+    }
     if (tpr <= 0 || tpr > q4 || q4 % tpr || q4 / tpr > 8) tpr = q4 < 8 ? q4 : 8;
     int lg = 0;
     while ((1 << lg) < tpr) ++lg;
@@ -873,7 +953,6 @@ cudaError_t spmm_pk32(const unsigned *pk, int n, const float *x, float *y, int n
     const long long work = (long long)n * tpr;
     if (work >= (1LL << 31)) return cudaErrorInvalidValue;
     const unsigned blocks = (unsigned)((work + TB - 1) / TB);
-    const uint4 *p4 = (const uint4 *)pk;
     switch (q4 / tpr) {
     case 1: k_spmm_pk<1><<<blocks, TB, 0, s>>>(p4, n, (const float4 *)x, (float4 *)y, q4, lg); break;
     case 2: k_spmm_pk<2><<<blocks, TB, 0, s>>>(p4, n, (const float4 *)x, (float4 *)y, q4, lg); break;

@@ -85,7 +85,8 @@ bool tune_get_spmm(int n, int nv, int *tpr) {
 
 void tune_set_spmm(int n, int nv, int tpr) {
     std::lock_guard<std::mutex> g(g_mu);
-    g_spmm[{n, nv_bucket(nv)}] = tpr;
+    if (tpr) g_spmm[{n, nv_bucket(nv)}] = tpr;
+    else g_spmm.erase({n, nv_bucket(nv)});
 }
 
 void tune_clear() {

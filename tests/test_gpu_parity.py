@@ -198,3 +198,25 @@ def test_barvortex_boundary_and_forcing(level, precision, golden):
     BW = np.stack([np.zeros_like(bw), np.zeros_like(bw), bw])
     out = bv.calc_batch(U, BU, BW, forcing=g["out_bv_bf_forcing0"])
     assert rel(out[2], g["out_bv_bf_step1"]) <= tol
+
+
+@pytest.mark.parametrize("level,nv", [(3, 128), (3, 256), (4, 128), (5, 128), (6, 32), (6, 64), (6, 256)])
+@pytest.mark.parametrize("special", [False, True])
+def test_interleaved_apply_of_long_rows_equals_the_short_rows_product(level, nv, special):
+    # 16 members at a time take the scattered kernel: the same sums in the same order, so the same bits;
+    # sizes where ranges are shorter than a pass (level 3), end within one, and hold one slice or several
+    torch = pytest.importorskip("torch")
+    m = phelm.Mesh.sphere(level)
+    ops = phelm.Operators(m, phelm.PHG_MIXED, tol=1e-12)
+    n = m.inner_size
+    x = torch.randn((n, nv), generator=torch.Generator(device="cuda").manual_seed(level), device="cuda")
+    if special:
+        x[n // 3, 5], x[n - 1, nv - 1], x[0, 0], x[n // 2, nv // 2] = float("inf"), float("-inf"), float("nan"), 3e38
+    y, z = torch.full_like(x, 7.0), torch.empty((n, 16), device="cuda")
+    for name in ("lapl", "idt"):
+        ops.mult32(name, x, y)
+        for k in range(0, nv, 16):
+            ops.mult32(name, x[:, k:k + 16].contiguous(), z)
+            assert torch.equal(torch.nan_to_num(y[:, k:k + 16], 1.25, 2e38, -2e38),
+                               torch.nan_to_num(z, 1.25, 2e38, -2e38))
+            assert torch.equal(torch.isnan(y[:, k:k + 16]), torch.isnan(z))
