@@ -59,7 +59,10 @@ constexpr int LS_MIN_TUNED = 8;  // the fewest right-hand sides for which the au
 // block, the former win once the vectors outgrow that -- by rows x right-hand
 // sides, from about these products on (measured; see choose_path)
 constexpr long long LS_MIN_WORK = 8000000;    // Chebyshev solves
-constexpr long long LSG_MIN_WORK = 2000000;   // multigrid Laplacians
+// multigrid Laplacians (above level 5 the lockstep path runs a cycle more), and
+// the fewest right-hand sides
+constexpr long long LSG_MIN_WORK = 1100000, LSG_MIN_WORK_L6 = 1500000;
+constexpr int LSG_MIN_NV = 16;
 
 // One operator's share of a multi-operator launch (meshes of several levels
 // in one persistent launch): right-hand sides [v0, next v0) use this
@@ -1349,61 +1352,79 @@ __global__ void __launch_bounds__(256) k_ls_sq(const double *__restrict__ A, int
 }
 
 // ||r||^2 and ||b||^2 of every member: the sums of its nbx block partials
-// (one warp per member, fixed order)
+// (one warp per member, fixed order).  With beta set: ||r||, the scale 1 / ||r||
+// (0 once converged) and, in nrm[2 v], ||r|| / ||b||, by eight lanes of a block:
+// all on one SM, as part of the stopping test, the roots and quotients of
+// 2,048 members took 56 us of its FP64 pipe (20 us now).
 __global__ void __launch_bounds__(256) k_ls_nrm(const double *rpart, const double *bpart, int nbx, double *nrm,
-                                                int nv, const int *done) {
+                                                int nv, const int *done, double tol = 0.0, double *beta = nullptr,
+                                                double *sc = nullptr) {
     if (*(volatile const int *)done) return;
-    const int v = blockIdx.x * NWARP + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-    if (v >= nv) return;
-    double tr = 0.0, tb = 0.0;
-    for (int q = lane; q < nbx; q += 32) {
-        tr += rpart[(size_t)v * nbx + q];
-        tb += bpart[(size_t)v * nbx + q];
+    __shared__ double sums[NWARP][2];
+    const int wp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    int v = blockIdx.x * NWARP + wp;
+    if (v < nv) {
+        double tr = 0.0, tb = 0.0;
+        for (int q = lane; q < nbx; q += 32) {
+            tr += rpart[(size_t)v * nbx + q];
+            tb += bpart[(size_t)v * nbx + q];
+        }
+        tr = warp_sum(tr);
+        tb = warp_sum(tb);
+        if (lane == 0) {
+            if (beta) { sums[wp][0] = tr; sums[wp][1] = tb; }
+            else { nrm[2 * v] = tr; nrm[2 * v + 1] = tb; }
+        }
     }
-    tr = warp_sum(tr);
-    tb = warp_sum(tb);
-    if (lane == 0) { nrm[2 * v] = tr; nrm[2 * v + 1] = tb; }
+    if (!beta) return;
+    __syncthreads();
+    v = blockIdx.x * NWARP + threadIdx.x;
+    if (threadIdx.x < NWARP && v < nv) {
+        const double bt = sqrt(sums[threadIdx.x][0]), bn = sqrt(sums[threadIdx.x][1]);
+        const double rel = bn > 0.0 ? bt / bn : 0.0;
+        nrm[2 * v] = rel;
+        beta[v] = bt;
+        sc[v] = rel <= tol || bt == 0.0 ? 0.0 : 1.0 / bt;
+    }
 }
 
-// per-member scales 1/||r|| (0 once converged), the stopping test and the stats
-// The cycle's steps (*kc): K, or fewer when every open member needs a smaller
-// reduction (tol / rel, factor 2 margin; steps for a reduction eps:
-// ceil((lg - log eps) / ls) + 1), rounded up to K's parity so that the
-// iterate ends in the buffer the K-step sequence ends in.
+// the stopping test and the stats
+// The cycle's steps (*kc): K, or fewer when the open member with the largest
+// residual needs a smaller reduction (tol / rel, factor 2 margin; steps for a
+// reduction eps: ceil((lg - log eps) / ls) + 1), rounded up to K's parity so
+// that the iterate ends in the buffer the K-step sequence ends in.
 __global__ void __launch_bounds__(256) k_ls_scale(const double *nrm, int nv, int nvp, double tol, double *beta,
                                                   double *sc, int *done, GmresStats *st, int cycle, int K,
                                                   double bytes, double lg, double ls, int *kc) {
     if (*(volatile int *)done) return;
     __shared__ double rmax[NWARP];
-    __shared__ int open[NWARP], kneed[NWARP];
-    double mx = 0.0;
-    int op = 0, kn = 2;
+    __shared__ int open[NWARP];
+    __shared__ double rneed[NWARP];
+    double mx = 0.0, worst = 0.0;   // over all members, over the open ones
+    int op = 0;
     for (int v = threadIdx.x; v < nvp; v += blockDim.x) {
         if (v >= nv) { sc[v] = 0.0; beta[v] = 0.0; continue; }
-        const double bt = sqrt(nrm[2 * v]), bn = sqrt(nrm[2 * v + 1]);
-        const double rel = bn > 0.0 ? bt / bn : 0.0;
-        const bool conv = rel <= tol || bt == 0.0;
-        beta[v] = bt;
-        sc[v] = conv ? 0.0 : 1.0 / bt;
+        const double rel = nrm[2 * v];
         mx = max_nan(mx, rel);
         if (!(rel == rel)) mx = rel;   // NaN propagates into the stats
-        op += conv ? 0 : 1;
-        if (!conv) {
-            const double need = ls > 0.0 ? (lg + log(2.0 * rel / tol)) / ls : (double)K;
-            kn = need + 1.0 < (double)K ? max(kn, (int)ceil(need) + 1) : K;   // NaN: K
-        }
+        if (!(rel <= tol || beta[v] == 0.0)) { ++op; worst = max_nan(worst, rel); }
     }
     for (int o = 16; o > 0; o >>= 1) {
         mx = max_nan(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+        worst = max_nan(worst, __shfl_xor_sync(0xffffffffu, worst, o));
         op += __shfl_xor_sync(0xffffffffu, op, o);
-        kn = max(kn, __shfl_xor_sync(0xffffffffu, kn, o));
     }
-    if ((threadIdx.x & 31) == 0) { rmax[threadIdx.x >> 5] = mx; open[threadIdx.x >> 5] = op; kneed[threadIdx.x >> 5] = kn; }
+    if ((threadIdx.x & 31) == 0) { rmax[threadIdx.x >> 5] = mx; open[threadIdx.x >> 5] = op; rneed[threadIdx.x >> 5] = worst; }
     __syncthreads();
     if (threadIdx.x == 0) {
         double m = 0.0;
         int o = 0, k = 2;
-        for (int w = 0; w < NWARP; ++w) { m = max_nan(m, rmax[w]); o += open[w]; k = max(k, kneed[w]); }
+        worst = 0.0;
+        for (int w = 0; w < NWARP; ++w) { m = max_nan(m, rmax[w]); o += open[w]; worst = max_nan(worst, rneed[w]); }
+        if (o) {
+            const double need = ls > 0.0 ? (lg + log(2.0 * worst / tol)) / ls : (double)K;
+            k = need + 1.0 < (double)K ? max(k, (int)ceil(need) + 1) : K;   // NaN: K
+        }
         k = min(K, k + ((K - k) & 1));
         if (cycle == 0) st->steps_total = 0;
         else st->steps_total += *kc;   // the previous cycle's steps
@@ -1648,7 +1669,7 @@ cudaError_t cheb_lockstep(const DevSolveOp &op, const double *B, double *X, int 
         case 7: k_ls_resid<7><<<rblocks, 256, 0, s>>>(op.A.col, op.A.val, n, B, X, ld, R, nv, rpart, nbx, done); break;
         default: k_ls_resid<8><<<rblocks, 256, 0, s>>>(op.A.col, op.A.val, n, B, X, ld, R, nv, rpart, nbx, done); break;
         }
-        k_ls_nrm<<<(nv + NWARP - 1) / NWARP, 256, 0, s>>>(rpart, bpart, nbx, nrm, nv, done);
+        k_ls_nrm<<<(nv + NWARP - 1) / NWARP, 256, 0, s>>>(rpart, bpart, nbx, nrm, nv, done, tol, beta, sc);
         k_ls_scale<<<1, 256, 0, s>>>(nrm, nv, nvp, tol, beta, sc, done, st, c, K, c ? cyc : 0.0, lg, ls, kcp);
         if (c == LS_MAXC) break;
         k_ls_init<<<capped(ntile, cap_init), 256, 0, s>>>(R, n, nv, nvp, sc, op.dinv32, (float)pl.c0, rv, e0,
@@ -1707,31 +1728,25 @@ int env_int(const char *name, int dflt) {
 // index range with a grid-stride loop over a grid capped at a few blocks per
 // SM, so a launch that finds its flag set costs little.
 constexpr int LSG_M = 8;        // Arnoldi steps per refinement cycle
-// refinement cycles at most: three cycles of an 1e-5 inner reduction reach
-// 1e-12 from a zero start; a fourth only added skipped launches (L6 x 32
-// ensemble step 22.5 -> 21.9 ms without it)
-constexpr int LSG_MAXC = 3;
+// refinement cycles at most: three of eight steps reach 1e-12 from a zero start
+// up to level 5 and stop at 1e-11 on level 6, where a fourth takes all right-hand
+// sides there; below it would only add skipped launches (level 5 x 256 solves
+// 3.4 -> 4.0 ms)
+inline int lsg_cycles(int n) { return n > 20000 ? 4 : 3; }
 constexpr int LSG_MINRHS = 8;   // fewest right-hand sides the path accepts
 constexpr int LSG_SMALL = 700;  // levels of at most this many rows run in one shared-memory kernel
-constexpr size_t LSG_SMALL_SMEM = 160 * 1024;
 
-struct LsgLevel {               // one multigrid level; buffers n x nvp FP32
-    int n, W, Wr;
-    const int *col; const float *a; const float *d;
-    const int *pc; const float *pw;      // prolongation from level + 1
-    const int *rf; const float *rw;      // restriction to level + 1
-    float *x, *xo, *r, *b;
+struct LsgLevel {               // one multigrid level: its composed operators; vectors n x nvp FP32
+    int n;
+    const int *qc, *tc, *uc;
+    const float *qv, *tv, *uv;
+    float *x, *b;               // below the finest level
 };
 
 struct LsgParams {
-    int n, nv, nvp, q4, m, nlev, W, RB, nbx, ld, max_iter, maxc;
+    int n, nv, nvp, q4, m, W, RB, nbx, ld, max_iter, maxc;
     double tol, inner_rtol, step_row_bytes, resid_row_bytes;
-    float omega;
     const int *col; const float *a32;    // fine operator, FP32 (w = A z)
-    LsgLevel lev[MG_MAXLEV];
-    int nc; const float *cinv;           // coarsest level, dense inverse
-    int lc;                              // levels [lc, nlev) run in one kernel, in shared memory
-    LsgLevel *levs;                      // device copy of lev[] (indexed at run time by that kernel)
     const double *B; double *X;          // member-major FP64, leading dimension ld
     float *V, *Z, *w;                    // (m + 1), m and 1 interleaved vectors
     double *R, *rpart, *bpart, *nrm;     // FP64 residual, norm partials, norms (2 per member)
@@ -1867,288 +1882,178 @@ __device__ __forceinline__ bool lsg_skip(const LsgParams &P, int j) {
 
 __device__ __forceinline__ float4 f4mul(float4 a, float4 b) { return make_float4(a.x * b.x, a.y * b.y, a.z * b.z, a.w * b.w); }
 
-// down sweep at level l: x = w D^-1 b, r = b - A x (from b alone).  With
-// vout set, b = src * vscale (the Krylov vector v_j = w / ||w|| formed on the
-// fly from the previous step's w) and the block's own rows of v_j are stored.
-__global__ void __launch_bounds__(256) k_mg_down(LsgParams P, LsgLevel L, const float *src, float *vout, int j) {
-    if (lsg_skip(P, j)) return;
-    const int q4 = P.q4;
-    const float4 *b = (const float4 *)src;
-    float4 *x = (float4 *)L.x, *r = (float4 *)L.r;
-    const float om = P.omega;
-    const long long total = (long long)L.n * q4;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += lsg_grid_stride()) {
-        const int i = (int)(t / q4), q = (int)(t - (long long)i * q4);
-        const float4 sc = vout ? ((const float4 *)P.vscale)[q] : make_float4(1.f, 1.f, 1.f, 1.f);
-        int c[8];
-        float a[8];
-        float4 g[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-            if (k < L.W) { c[k] = __ldg(&L.col[(size_t)k * L.n + i]); a[k] = __ldg(&L.a[(size_t)k * L.n + i]); }
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-            if (k < L.W) g[k] = f4mul(b[(size_t)c[k] * q4 + q], sc);
-        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-            if (k < L.W) s = f4fma(a[k] * (om * __ldg(&L.d[c[k]])), g[k], s);
-        const float4 bi = f4mul(b[(size_t)i * q4 + q], sc);
-        if (vout) ((float4 *)vout)[(size_t)i * q4 + q] = bi;
-        const float di = om * __ldg(&L.d[i]);
-        x[(size_t)i * q4 + q] = make_float4(di * bi.x, di * bi.y, di * bi.z, di * bi.w);
-        r[(size_t)i * q4 + q] = make_float4(bi.x - s.x, bi.y - s.y, bi.z - s.z, bi.w - s.w);
-    }
-}
-
-// b_{l+1} = R r_l
-__global__ void __launch_bounds__(256) k_mg_restrict(LsgParams P, LsgLevel L, LsgLevel C, int j) {
-    if (lsg_skip(P, j)) return;
-    const int q4 = P.q4, nc = C.n;
-    const float4 *r = (const float4 *)L.r;
-    float4 *bc = (float4 *)C.b;
-    const long long total = (long long)nc * q4;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += lsg_grid_stride()) {
-        const int cc = (int)(t / q4), q = (int)(t - (long long)cc * q4);
-        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int k = 0; k < L.Wr; ++k) {
-            const int f = __ldg(&L.rf[(size_t)k * nc + cc]);
-            if (f >= 0) s = f4fma(__ldg(&L.rw[(size_t)k * nc + cc]), r[(size_t)f * q4 + q], s);
-        }
-        bc[(size_t)cc * q4 + q] = s;
-    }
-}
-
-// threads of a k_mg_small block: one per row of the 641-row level (a block runs
-// one 4-member chunk alone, so the small levels' sweeps are its latency)
+// threads of a k_lsg_small block: one per row of the 641-row level (a block runs
+// one 4-member chunk alone, so the small levels' phases are its latency)
 constexpr int MG_SMALL_TB = 1024;
 
-// Levels [lc, nlev) for one 4-member chunk per block, in shared memory (four
-// float4 vectors per level: x, t, b, r): b_lc = R r_{lc-1} (or the input when
-// lc = 0), down sweeps and restrictions, the dense coarsest solve, the
-// prolongations and up sweeps; x_lc is written to out (the coarse correction
-// of level lc - 1, or the V-cycle's output when lc = 0).  Replaces one launch
-// per small level and phase by a single launch.
-__global__ void __launch_bounds__(MG_SMALL_TB) k_mg_small(LsgParams P, const float *src, float *vout, float *out, int j) {
+// The V-cycle as composed operators (phg_mgplan.cpp: b' = Q b, x = T b + U x'):
+// one gather per level down and one up where its sweeps took a down pass, a
+// restriction, a prolongation and a smoothing, each a launch that read and
+// wrote whole vectors.  At level 0 b is the Krylov vector
+// w / ||w|| of the previous step, scaled after the sum; the way up stores it.
+// What bounds these launches is L2 (a level-5 vector of 256 members is 10 MB):
+// a V-cycle 86 -> 41 us there, the step of 256 members 30.7 -> 27.0 ms with
+// the fused product and dots.
+
+// the sum of K entries of a row's table times rows of x
+template <int K>
+__device__ __forceinline__ float4 row_product(const int *__restrict__ col, const float *__restrict__ val, int row,
+                                              const float4 *x, unsigned q4, unsigned q, float4 s) {
+    unsigned c[K];
+    float4 g[K];
+    float a[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) { c[k] = __ldg(&col[row * K + k]); a[k] = __ldg(&val[row * K + k]); }
+#pragma unroll
+    for (int k = 0; k < K; ++k) g[k] = x[c[k] * q4 + q];   // n q4 < 2^31 (host check)
+#pragma unroll
+    for (int k = 0; k < K; ++k) s = f4fma(a[k], g[k], s);
+    return s;
+}
+// Q's twenty entries in two batches: forty gathers' registers would halve the blocks per SM
+__device__ __forceinline__ float4 q_product(const LsgLevel &L, int row, const float4 *x, unsigned q4, unsigned q) {
+    static_assert(MGX_WQ == 20, "two batches of ten");
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int *c = L.qc + row * MGX_WQ;
+    const float *v = L.qv + row * MGX_WQ;
+    s = row_product<10>(c, v, 0, x, q4, q, s);
+    return row_product<10>(c + 10, v + 10, 0, x, q4, q, s);
+}
+
+__global__ void __launch_bounds__(256) k_lsg_q(LsgParams P, LsgLevel L, int nc, const float *src, int scaled, float *dst,
+                                               int j) {
+    if (lsg_skip(P, j)) return;
+    const unsigned q4 = P.q4, total = nc * q4;
+    for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += lsg_grid_stride()) {
+        const unsigned c = t / q4, q = t - c * q4;
+        float4 s = q_product(L, c, (const float4 *)src, q4, q);
+        if (scaled) s = f4mul(s, ((const float4 *)P.vscale)[q]);
+        ((float4 *)dst)[t] = s;
+    }
+}
+
+// x = T b + U x'; with vout set b = src * vscale, and the rows of v_j are stored
+__global__ void __launch_bounds__(256) k_lsg_up(LsgParams P, LsgLevel L, const float *src, float *vout, const float *xc,
+                                                float *out, int j) {
+    if (lsg_skip(P, j)) return;
+    const unsigned q4 = P.q4, total = L.n * q4;
+    for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < total; t += lsg_grid_stride()) {
+        const unsigned i = t / q4, q = t - i * q4;
+        const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+        float4 s = row_product<MGX_WT>(L.tc, L.tv, i, (const float4 *)src, q4, q, z);
+        const float4 u = row_product<MGX_WU>(L.uc, L.uv, i, (const float4 *)xc, q4, q, z);
+        if (vout) {
+            const float4 sc = ((const float4 *)P.vscale)[q];
+            s = f4mul(s, sc);
+            ((float4 *)vout)[t] = f4mul(((const float4 *)src)[t], sc);
+        }
+        ((float4 *)out)[t] = make_float4(s.x + u.x, s.y + u.y, s.z + u.z, s.w + u.w);
+    }
+}
+
+// Levels [lc, nlev) for one 4-member chunk per block: b' = Q b_lc, x' = B b'
+// with the levels from lc + 1 down as one dense matrix, x_lc = T b_lc + U x'.
+// Three dependent phases where sweeps through the levels were a dozen (level 5
+// x 256: 18.2 -> 13.4 us with b_lc's own gather in it, which as a launch of
+// its own reads whole rows instead of 16 bytes of each: solves -3 %).
+__global__ void __launch_bounds__(MG_SMALL_TB) k_lsg_small(LsgParams P, LsgLevel L, int n1, const float *dense,
+                                                           const float *src, float *vout, float *out, int j) {
     if (lsg_skip(P, j)) return;
     extern __shared__ float4 sm4[];
-    const int q4 = P.q4, lc = P.lc, last = P.nlev - 1;
-    const float om = P.omega;
-    const LsgLevel *LV = P.levs;
+    const int q4 = P.q4, n = L.n, st = mgx_stride(n1);
+    float4 *b = sm4, *b1 = b + n, *x1 = b1 + st;
     for (int q = blockIdx.x; q < q4; q += gridDim.x) {
-        // shared-memory offsets of the levels
-        int off[MG_MAXLEV];
-        int o = 0;
-        for (int l = lc; l <= last; ++l) { off[l] = o; o += 4 * LV[l].n; }
-        // b at level lc
-        {
-            const LsgLevel L = LV[lc];
-            float4 *b = sm4 + off[lc] + 2 * L.n;
-            if (lc == 0) {
-                const float4 sc = vout ? ((const float4 *)P.vscale)[q] : make_float4(1.f, 1.f, 1.f, 1.f);
-                for (int i = threadIdx.x; i < L.n; i += blockDim.x) {
-                    const float4 v = f4mul(((const float4 *)src)[(size_t)i * q4 + q], sc);
-                    b[i] = v;
-                    if (vout) ((float4 *)vout)[(size_t)i * q4 + q] = v;
-                }
-            } else {
-                const LsgLevel F = LV[lc - 1];
-                const float4 *r = (const float4 *)F.r;
-                for (int c = threadIdx.x; c < L.n; c += blockDim.x) {
-                    float4 sacc = make_float4(0.f, 0.f, 0.f, 0.f);
-                    for (int k = 0; k < F.Wr; ++k) {
-                        const int f = __ldg(&F.rf[(size_t)k * L.n + c]);
-                        if (f >= 0) sacc = f4fma(__ldg(&F.rw[(size_t)k * L.n + c]), r[(size_t)f * q4 + q], sacc);
-                    }
-                    b[c] = sacc;
-                }
-            }
+        const float4 sc = vout ? ((const float4 *)P.vscale)[q] : make_float4(1.f, 1.f, 1.f, 1.f);
+        for (int i = threadIdx.x; i < n; i += MG_SMALL_TB) {
+            const float4 v = f4mul(((const float4 *)src)[i * q4 + q], sc);
+            b[i] = v;
+            if (vout) ((float4 *)vout)[i * q4 + q] = v;
         }
         __syncthreads();
-        // down: x = w D^-1 b, r = b - A x, b_{l+1} = R r
-        for (int l = lc; l < last; ++l) {
-            const LsgLevel L = LV[l];
-            float4 *x = sm4 + off[l], *b = x + 2 * L.n, *r = x + 3 * L.n;
-            for (int i = threadIdx.x; i < L.n; i += blockDim.x) {
-                const float di = om * __ldg(&L.d[i]);
-                x[i] = make_float4(di * b[i].x, di * b[i].y, di * b[i].z, di * b[i].w);
+        for (int i = threadIdx.x; i < st; i += MG_SMALL_TB)
+            b1[i] = i < n1 ? q_product(L, i, b, 1, 0) : make_float4(0.f, 0.f, 0.f, 0.f);
+        __syncthreads();
+        for (int i = threadIdx.x >> 2; i < n1; i += MG_SMALL_TB / 4) {   // four lanes a row
+            const float4 *B = (const float4 *)(dense + i * st);
+            const int h = threadIdx.x & 3;
+            float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int k = h; k < st / 4; k += 4) {
+                const float4 a = __ldg(&B[k]);
+                s = f4fma(a.x, b1[4 * k], s); s = f4fma(a.y, b1[4 * k + 1], s);
+                s = f4fma(a.z, b1[4 * k + 2], s); s = f4fma(a.w, b1[4 * k + 3], s);
             }
-            __syncthreads();
-            for (int i = threadIdx.x; i < L.n; i += blockDim.x) {
-                float4 sacc = make_float4(0.f, 0.f, 0.f, 0.f);
-                for (int k = 0; k < L.W; ++k)
-                    sacc = f4fma(__ldg(&L.a[(size_t)k * L.n + i]), x[__ldg(&L.col[(size_t)k * L.n + i])], sacc);
-                r[i] = make_float4(b[i].x - sacc.x, b[i].y - sacc.y, b[i].z - sacc.z, b[i].w - sacc.w);
+            const unsigned m = 0xfu << (threadIdx.x & 28);
+            for (int o = 1; o < 4; o *= 2) {
+                s.x += __shfl_xor_sync(m, s.x, o); s.y += __shfl_xor_sync(m, s.y, o);
+                s.z += __shfl_xor_sync(m, s.z, o); s.w += __shfl_xor_sync(m, s.w, o);
             }
-            __syncthreads();
-            const LsgLevel C = LV[l + 1];
-            float4 *bc = sm4 + off[l + 1] + 2 * C.n;
-            for (int c = threadIdx.x; c < C.n; c += blockDim.x) {
-                float4 sacc = make_float4(0.f, 0.f, 0.f, 0.f);
-                for (int k = 0; k < L.Wr; ++k) {
-                    const int f = __ldg(&L.rf[(size_t)k * C.n + c]);
-                    if (f >= 0) sacc = f4fma(__ldg(&L.rw[(size_t)k * C.n + c]), r[f], sacc);
-                }
-                bc[c] = sacc;
-            }
-            __syncthreads();
+            if (h == 0) x1[i] = s;
         }
-        // coarsest: x = C^-1 b
-        {
-            const int n = P.nc;
-            float4 *x = sm4 + off[last], *b = x + 2 * n;
-            for (int i = threadIdx.x; i < n; i += blockDim.x) {
-                float4 sacc = make_float4(0.f, 0.f, 0.f, 0.f);
-                for (int k = 0; k < n; ++k) sacc = f4fma(__ldg(&P.cinv[(size_t)i * n + k]), b[k], sacc);
-                x[i] = sacc;
-            }
-            __syncthreads();
+        __syncthreads();
+        for (int i = threadIdx.x; i < n; i += MG_SMALL_TB) {
+            const float4 s = row_product<MGX_WT>(L.tc, L.tv, i, b, 1, 0, make_float4(0.f, 0.f, 0.f, 0.f));
+            ((float4 *)out)[i * q4 + q] = row_product<MGX_WU>(L.uc, L.uv, i, x1, 1, 0, s);
         }
-        // up: x += P x_{l+1}; x = x + w D^-1 (b - A x)
-        for (int l = last - 1; l >= lc; --l) {
-            const LsgLevel L = LV[l];
-            float4 *x = sm4 + off[l], *t = x + L.n, *b = x + 2 * L.n;
-            const float4 *xc = sm4 + off[l + 1];
-            for (int i = threadIdx.x; i < L.n; i += blockDim.x) {
-                const int c0 = __ldg(&L.pc[2 * i]), c1 = __ldg(&L.pc[2 * i + 1]);
-                float4 sacc = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (c0 >= 0) sacc = f4fma(__ldg(&L.pw[2 * i]), xc[c0], sacc);
-                if (c1 >= 0) sacc = f4fma(__ldg(&L.pw[2 * i + 1]), xc[c1], sacc);
-                x[i] = make_float4(x[i].x + sacc.x, x[i].y + sacc.y, x[i].z + sacc.z, x[i].w + sacc.w);
-            }
-            __syncthreads();
-            for (int i = threadIdx.x; i < L.n; i += blockDim.x) {
-                float4 sacc = make_float4(0.f, 0.f, 0.f, 0.f);
-                for (int k = 0; k < L.W; ++k)
-                    sacc = f4fma(__ldg(&L.a[(size_t)k * L.n + i]), x[__ldg(&L.col[(size_t)k * L.n + i])], sacc);
-                const float di = om * __ldg(&L.d[i]);
-                t[i] = make_float4(x[i].x + di * (b[i].x - sacc.x), x[i].y + di * (b[i].y - sacc.y),
-                                   x[i].z + di * (b[i].z - sacc.z), x[i].w + di * (b[i].w - sacc.w));
-            }
-            __syncthreads();
-            float4 *dst = l == lc ? (float4 *)out : x;
-            if (l == lc)
-                for (int i = threadIdx.x; i < L.n; i += blockDim.x) dst[(size_t)i * q4 + q] = t[i];
-            else
-                for (int i = threadIdx.x; i < L.n; i += blockDim.x) x[i] = t[i];
-            __syncthreads();
-        }
-        if (lc == last)   // the whole cycle is the dense solve
-            for (int i = threadIdx.x; i < P.nc; i += blockDim.x) ((float4 *)out)[(size_t)i * q4 + q] = sm4[off[last] + i];
         __syncthreads();
     }
 }
 
-// copy of the level descriptors into device memory (static indices only)
-__global__ void k_lsg_levels(LsgParams P) {
-    if (threadIdx.x || blockIdx.x) return;
+// w = A z_j (fine operator, FP32) and the partials of its products with the
+// basis: dpart[rb][l][v] = sum over the block's rows of V_l[r][v] w[r][v],
+// l <= j (grid RB x nvp/32; eight lanes hold a row's 32 members, a warp four
+// rows).  One launch and w not read back, where the product and the dots were
+// two; sixteen bytes per load: level 5 x 256, on average over a cycle's steps,
+// 35 -> 19 us.
+__global__ void __launch_bounds__(256) k_lsg_spmm_dot(LsgParams P, int j) {
+    if (lsg_skip(P, j)) return;
+    __shared__ float4 red[NWARP][LSG_M][8];
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, n = P.n, W = P.W;
+    const unsigned q4 = P.q4, q = blockIdx.y * 8 + (lane & 7);
+    const float4 *z = (const float4 *)P.Z + (size_t)j * n * q4 + q, *V = (const float4 *)P.V + q;
+    float4 *w = (float4 *)P.w + q;
+    const int rpr = (n + P.RB - 1) / P.RB;
+    const int r0 = min(n, (int)blockIdx.x * rpr), r1 = min(n, r0 + rpr);
+    const size_t vs = (size_t)n * q4;
+    float4 t[LSG_M];
 #pragma unroll
-    for (int k = 0; k < MG_MAXLEV; ++k) P.levs[k] = P.lev[k];
-}
-
-// x_l += P x_{l+1}
-__global__ void __launch_bounds__(256) k_mg_prolong(LsgParams P, LsgLevel L, const float *xcoarse, int j) {
-    if (lsg_skip(P, j)) return;
-    const int q4 = P.q4;
-    const float4 *xc = (const float4 *)xcoarse;
-    float4 *x = (float4 *)L.x;
-    const long long total = (long long)L.n * q4;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += lsg_grid_stride()) {
-        const int i = (int)(t / q4), q = (int)(t - (long long)i * q4);
-        const int c0 = __ldg(&L.pc[2 * i]), c1 = __ldg(&L.pc[2 * i + 1]);
-        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (c0 >= 0) s = f4fma(__ldg(&L.pw[2 * i]), xc[(size_t)c0 * q4 + q], s);
-        if (c1 >= 0) s = f4fma(__ldg(&L.pw[2 * i + 1]), xc[(size_t)c1 * q4 + q], s);
-        float4 xi = x[(size_t)i * q4 + q];
-        x[(size_t)i * q4 + q] = make_float4(xi.x + s.x, xi.y + s.y, xi.z + s.z, xi.w + s.w);
-    }
-}
-
-// post-smoothing at level l: out = x + w D^-1 (b - A x)
-__global__ void __launch_bounds__(256) k_mg_smooth(LsgParams P, LsgLevel L, const float *bsrc, float *out, int j) {
-    if (lsg_skip(P, j)) return;
-    const int q4 = P.q4;
-    const float4 *b = (const float4 *)bsrc, *x = (const float4 *)L.x;
-    float4 *o = (float4 *)out;
-    const float om = P.omega;
-    const long long total = (long long)L.n * q4;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += lsg_grid_stride()) {
-        const int i = (int)(t / q4), q = (int)(t - (long long)i * q4);
-        int c[8];
-        float a[8];
+    for (int l = 0; l < LSG_M; ++l) t[l] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int r = r0 + 4 * wp + (lane >> 3); r < r1; r += 4 * NWARP) {
         float4 g[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-            if (k < L.W) { c[k] = __ldg(&L.col[(size_t)k * L.n + i]); a[k] = __ldg(&L.a[(size_t)k * L.n + i]); }
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-            if (k < L.W) g[k] = x[(size_t)c[k] * q4 + q];
-        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-            if (k < L.W) s = f4fma(a[k], g[k], s);
-        const float4 bi = b[(size_t)i * q4 + q], xi = x[(size_t)i * q4 + q];
-        const float di = om * __ldg(&L.d[i]);
-        o[(size_t)i * q4 + q] = make_float4(xi.x + di * (bi.x - s.x), xi.y + di * (bi.y - s.y),
-                                            xi.z + di * (bi.z - s.z), xi.w + di * (bi.w - s.w));
-    }
-}
-
-// w = A z_j (fine operator, FP32)
-__global__ void __launch_bounds__(256) k_lsg_spmm(LsgParams P, int j) {
-    if (lsg_skip(P, j)) return;
-    const int q4 = P.q4, n = P.n, W = P.W;
-    const float4 *z = (const float4 *)(P.Z + (size_t)j * n * P.nvp);
-    float4 *w = (float4 *)P.w;
-    const long long total = (long long)n * q4;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total; t += lsg_grid_stride()) {
-        const int i = (int)(t / q4), q = (int)(t - (long long)i * q4);
-        int c[8];
         float a[8];
-        float4 g[8];
 #pragma unroll
         for (int k = 0; k < 8; ++k)
-            if (k < W) { c[k] = __ldg(&P.col[(size_t)k * n + i]); a[k] = __ldg(&P.a32[(size_t)k * n + i]); }
-#pragma unroll
-        for (int k = 0; k < 8; ++k)
-            if (k < W) g[k] = z[(size_t)c[k] * q4 + q];
+            if (k < W) {
+                g[k] = z[(unsigned)__ldg(&P.col[(size_t)k * n + r]) * q4];
+                a[k] = __ldg(&P.a32[(size_t)k * n + r]);
+            }
         float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int k = 0; k < 8; ++k)
             if (k < W) s = f4fma(a[k], g[k], s);
-        w[(size_t)i * q4 + q] = s;
+        w[(unsigned)r * q4] = s;
+#pragma unroll
+        for (int l = 0; l < LSG_M; ++l)
+            if (l <= j) {
+                const float4 v = V[l * vs + (unsigned)r * q4];
+                t[l] = make_float4(fmaf(v.x, s.x, t[l].x), fmaf(v.y, s.y, t[l].y), fmaf(v.z, s.z, t[l].z),
+                                   fmaf(v.w, s.w, t[l].w));
+            }
     }
-}
-
-// dot partials: dpart[rb][l][v] = sum over the block's rows of V_l[r][v] w[r][v], l <= j
-// (grid RB x nvp/32; lane = member, warps stride the rows; eight vectors per pass)
-__global__ void __launch_bounds__(256) k_lsg_dot(LsgParams P, int j) {
-    if (lsg_skip(P, j)) return;
-    __shared__ double red[NWARP][8][32];
-    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-    const int v = blockIdx.y * 32 + lane, nvp = P.nvp, n = P.n;
-    const int rpr = (n + P.RB - 1) / P.RB;
-    const int r0 = min(n, (int)blockIdx.x * rpr), r1 = min(n, r0 + rpr);
-    const size_t vs = (size_t)n * nvp;
-    for (int l0 = 0; l0 <= j; l0 += 8) {
-        const int kk = min(8, j + 1 - l0);
-        float t[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        for (int r = r0 + wp; r < r1; r += NWARP) {
-            const float s = P.w[(size_t)r * nvp + v];
 #pragma unroll
-            for (int k = 0; k < 8; ++k)
-                if (k < kk) t[k] += P.V[(size_t)(l0 + k) * vs + (size_t)r * nvp + v] * s;
+    for (int l = 0; l < LSG_M; ++l)
+        if (l <= j) {
+            for (int o = 8; o < 32; o *= 2) {
+                t[l].x += __shfl_xor_sync(~0u, t[l].x, o); t[l].y += __shfl_xor_sync(~0u, t[l].y, o);
+                t[l].z += __shfl_xor_sync(~0u, t[l].z, o); t[l].w += __shfl_xor_sync(~0u, t[l].w, o);
+            }
+            if (lane < 8) red[wp][l][lane] = t[l];
         }
-#pragma unroll
-        for (int k = 0; k < 8; ++k) red[wp][k][lane] = (double)t[k];
-        __syncthreads();
-        for (int e = threadIdx.x; e < kk * 32; e += blockDim.x) {
-            const int k = e >> 5, ln = e & 31;
-            double s = 0.0;
-            for (int q = 0; q < NWARP; ++q) s += red[q][k][ln];
-            P.dpart[((size_t)blockIdx.x * (P.m + 1) + l0 + k) * nvp + blockIdx.y * 32 + ln] = s;
-        }
-        __syncthreads();
+    __syncthreads();
+    for (int e = threadIdx.x; e < (j + 1) * 32; e += blockDim.x) {
+        const int l = e >> 5, v = e & 31;
+        double s = 0.0;
+        for (int k = 0; k < NWARP; ++k) s += (double)((const float *)red[k][l])[v];
+        P.dpart[((size_t)blockIdx.x * (P.m + 1) + l) * P.nvp + blockIdx.y * 32 + v] = s;
     }
 }
 
@@ -2167,33 +2072,46 @@ __global__ void __launch_bounds__(256) k_lsg_hsum(LsgParams P, int j) {
     }
 }
 
-// w -= sum_l h_l V_l; ||w||^2 partials per row block
+// w -= sum_l h_l V_l; ||w||^2 partials per row block (lanes as k_lsg_spmm_dot;
+// 15.2 -> 12.4 us with 16-byte loads)
 __global__ void __launch_bounds__(256) k_lsg_update(LsgParams P, int j) {
     if (lsg_skip(P, j)) return;
-    __shared__ double red[NWARP][32];
-    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
-    const int v = blockIdx.y * 32 + lane, nvp = P.nvp, n = P.n;
+    __shared__ float4 red[NWARP][8];
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, n = P.n;
+    const unsigned q4 = P.q4, q = blockIdx.y * 8 + (lane & 7);
     const int rpr = (n + P.RB - 1) / P.RB;
     const int r0 = min(n, (int)blockIdx.x * rpr), r1 = min(n, r0 + rpr);
-    const size_t vs = (size_t)n * nvp;
-    float h[LSG_M];
+    const float4 *V = (const float4 *)P.V + q;
+    float4 *w = (float4 *)P.w + q;
+    const size_t vs = (size_t)n * q4;
+    float4 h[LSG_M];
 #pragma unroll
-    for (int l = 0; l < LSG_M; ++l) h[l] = (l <= j && v < P.nv) ? P.hv[(size_t)v * (P.m + 1) + l] : 0.f;
-    float a2 = 0.f;
-    for (int r = r0 + wp; r < r1; r += NWARP) {
-        float s = P.w[(size_t)r * nvp + v];
+    for (int l = 0; l < LSG_M; ++l) {
+        auto hv = [&](int k) { return l <= j && (int)(4 * q) + k < P.nv ? P.hv[(size_t)(4 * q + k) * (P.m + 1) + l] : 0.f; };
+        h[l] = make_float4(hv(0), hv(1), hv(2), hv(3));
+    }
+    float4 a2 = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int r = r0 + 4 * wp + (lane >> 3); r < r1; r += 4 * NWARP) {
+        float4 s = w[(unsigned)r * q4];
 #pragma unroll
         for (int l = 0; l < LSG_M; ++l)
-            if (l <= j) s -= h[l] * P.V[(size_t)l * vs + (size_t)r * nvp + v];
-        P.w[(size_t)r * nvp + v] = s;
-        a2 += s * s;
+            if (l <= j) {
+                const float4 v = V[l * vs + (unsigned)r * q4];
+                s.x -= h[l].x * v.x; s.y -= h[l].y * v.y; s.z -= h[l].z * v.z; s.w -= h[l].w * v.w;
+            }
+        w[(unsigned)r * q4] = s;
+        a2.x += s.x * s.x; a2.y += s.y * s.y; a2.z += s.z * s.z; a2.w += s.w * s.w;
     }
-    red[wp][lane] = (double)a2;
+    for (int o = 8; o < 32; o *= 2) {
+        a2.x += __shfl_xor_sync(~0u, a2.x, o); a2.y += __shfl_xor_sync(~0u, a2.y, o);
+        a2.z += __shfl_xor_sync(~0u, a2.z, o); a2.w += __shfl_xor_sync(~0u, a2.w, o);
+    }
+    if (lane < 8) red[wp][lane] = a2;
     __syncthreads();
     if (threadIdx.x < 32) {
         double s = 0.0;
-        for (int q = 0; q < NWARP; ++q) s += red[q][threadIdx.x];
-        P.npart[(size_t)blockIdx.x * nvp + blockIdx.y * 32 + threadIdx.x] = s;
+        for (int k = 0; k < NWARP; ++k) s += (double)((const float *)red[k])[threadIdx.x];
+        P.npart[(size_t)blockIdx.x * P.nvp + blockIdx.y * 32 + threadIdx.x] = s;
     }
 }
 
@@ -2286,7 +2204,7 @@ __global__ void __launch_bounds__(256) k_lsg_correct(LsgParams P) {
 
 struct LsgLayout {
     size_t V, Z, w, R, lev[MG_MAXLEV], rpart, bpart, nrm, dpart, npart, hcol, H, cs, sn, g, hv, yv;
-    size_t bnorm, beta_prev, target, relv, scale, vscale, ints, levs, total;
+    size_t bnorm, beta_prev, target, relv, scale, vscale, ints, total;
     int nvp, m, RB, nbx;
 };
 
@@ -2306,7 +2224,7 @@ LsgLayout lsg_layout(const DevSolveOp &op, int nv, int restart) {
     L.Z = o; o += m * vec;
     L.w = o; o += vec;
     L.R = o; o += al(8 * n * (size_t)nv);
-    for (int l = 0; l < op.mg.nlev && l < MG_MAXLEV; ++l) { L.lev[l] = o; o += 4 * al(4 * (size_t)op.mg.lev[l].n * nvp); }
+    for (int l = 1; l < op.mgx.nlev; ++l) { L.lev[l] = o; o += 2 * al(4 * (size_t)op.mgx.lev[l].n * nvp); }
     L.rpart = o; o += al(8 * (size_t)nv * L.nbx);
     L.bpart = o; o += al(8 * (size_t)nv * L.nbx);
     L.nrm = o; o += al(16 * nvp);
@@ -2326,87 +2244,52 @@ LsgLayout lsg_layout(const DevSolveOp &op, int nv, int restart) {
     L.scale = o; o += al(4 * nvp);
     L.vscale = o; o += al(4 * nvp);
     L.ints = o; o += al(4 * (6 * nvp + m + 2 + 1));
-    L.levs = o; o += al(sizeof(LsgLevel) * MG_MAXLEV);
     L.total = o;
     return L;
 }
 
+// the first level that k_lsg_small runs: of at most LSG_SMALL rows, and not the coarsest (-1: none)
+int lsg_small_level(const MgxDev &x) {
+    for (int l = 0; l + 1 < x.nlev; ++l)
+        if (x.lev[l].n <= LSG_SMALL) return l;
+    return -1;
+}
+
 bool lsg_applicable(const DevSolveOp &op, int nv, Precision p, int restart) {
     if (p != PREC_MIXED || !op.mgd || op.block4 || op.A.W > 8 || !op.a32 || nv < LSG_MINRHS || restart < 2) return false;
-    if (op.mg.nu1 != 1 || op.mg.nu2 != 1 || op.mg.nlev < 2 || op.mg.nlev > MG_MAXLEV || !op.mg.cinv32) return false;
-    for (int l = 0; l < op.mg.nlev; ++l) {
-        const MgLevelDev &D = op.mg.lev[l];
-        if (D.W > 8 || !D.a32 || !D.d32) return false;
-        if (l + 1 < op.mg.nlev && (!D.pc || !D.pw32 || !D.rf || !D.rw32)) return false;
-    }
+    const int lc = lsg_small_level(op.mgx);
+    if (lc < 0 || !op.mgx.B[lc + 1]) return false;
     return (long long)op.A.n * ((nv + 31) / 32 * 8) < (1LL << 31);
 }
 
-unsigned lsg_blocks(long long work, unsigned resident = 0) {
-    long long b = (work + 255) / 256;
-    long long cap = 4LL * sm_count();
-    if (resident > 0 && resident < cap) cap = resident;   // no partial second wave
-    if (b > cap) b = cap;
-    if (b < 1) b = 1;
-    return (unsigned)b;
-}
-
-// resident grids of the register-heavy lockstep multigrid kernels (80 registers:
-// 3 blocks of 256 threads per SM, fewer than the 4 per SM the other kernels
-// launch with), queried once at operator creation like ls_grids.  Capping
-// their grid at one resident wave instead of 4 blocks per SM avoids a second,
-// partial wave.
-struct LsgGrids {
-    unsigned down, smooth, spmm;
-};
-const LsgGrids &lsg_grids() {
-    static std::once_flag once;
-    static LsgGrids g;
-    std::call_once(once, [] {
-        g.down = resident_grid(k_mg_down, 0);
-        g.smooth = resident_grid(k_mg_smooth, 0);
-        g.spmm = resident_grid(k_lsg_spmm, 0);
-    });
-    return g;
+unsigned lsg_blocks(long long work) {
+    return (unsigned)std::max(1LL, std::min((work + 255) / 256, 4LL * sm_count()));
 }
 
 cudaError_t lsg_solve(const DevSolveOp &op, const double *B, double *X, int nv, int ld, int restart, int max_iter,
                       double tol, double inner_rtol, char *w, GmresStats *st, double mg_row_bytes, cudaStream_t s) {
-    const int lsg_maxc = LSG_MAXC;
+    const int lsg_maxc = lsg_cycles(op.A.n);
     const LsgLayout Lo = lsg_layout(op, nv, restart);
-    const int n = op.A.n, W = op.A.W, nvp = Lo.nvp, m = Lo.m, nlev = op.mg.nlev, last = nlev - 1;
+    const int n = op.A.n, W = op.A.W, nvp = Lo.nvp, m = Lo.m, lc = lsg_small_level(op.mgx);
     LsgParams P;
     memset(&P, 0, sizeof P);
-    P.n = n; P.nv = nv; P.nvp = nvp; P.q4 = nvp / 4; P.m = m; P.nlev = nlev; P.W = W; P.RB = Lo.RB; P.nbx = Lo.nbx;
+    P.n = n; P.nv = nv; P.nvp = nvp; P.q4 = nvp / 4; P.m = m; P.W = W; P.RB = Lo.RB; P.nbx = Lo.nbx;
     P.ld = ld; P.max_iter = max_iter; P.tol = tol; P.inner_rtol = inner_rtol;
     // algorithmic bytes per member and row (the per-member solver's model, FP32 vectors)
     P.step_row_bytes = W * 8.0 + 4.0 * 6.0 + mg_row_bytes;
     P.resid_row_bytes = W * 12.0 + 24.0;
-    P.omega = (float)op.mg.omega;
     P.col = op.A.col; P.a32 = op.a32;
-    for (int l = 0; l < nlev; ++l) {
-        const MgLevelDev &D = op.mg.lev[l];
-        LsgLevel &E = P.lev[l];
-        E.n = D.n; E.W = D.W; E.Wr = D.Wr; E.col = D.col; E.a = D.a32; E.d = D.d32;
-        E.pc = D.pc; E.pw = D.pw32; E.rf = D.rf; E.rw = D.rw32;
-        const size_t lv = (((size_t)D.n * nvp * 4) + 255) & ~size_t(255);
-        E.x = (float *)(w + Lo.lev[l]); E.xo = (float *)(w + Lo.lev[l] + lv);
-        E.r = (float *)(w + Lo.lev[l] + 2 * lv); E.b = (float *)(w + Lo.lev[l] + 3 * lv);
+    LsgLevel lev[MG_MAXLEV];
+    for (int l = 0; l <= lc; ++l) {
+        const MgxLevelDev &D = op.mgx.lev[l];
+        LsgLevel &E = lev[l];
+        E.n = D.n; E.qc = D.qc; E.tc = D.tc; E.uc = D.uc;
+        E.qv = (const float *)D.qv; E.tv = (const float *)D.tv; E.uv = (const float *)D.uv;
+        E.x = l ? (float *)(w + Lo.lev[l]) : nullptr;
+        E.b = l ? E.x + (Lo.lev[l + 1] - Lo.lev[l]) / 8 : nullptr;
     }
-    P.nc = op.mg.nc; P.cinv = op.mg.cinv32;
-    // the small levels: from the first with <= LSG_SMALL rows whose levels fit in shared memory
-    int lc = last;
-    for (int l = last; l >= 0; --l) {
-        size_t rows = 0;
-        for (int k = l; k <= last; ++k) rows += (size_t)op.mg.lev[k].n;
-        if (op.mg.lev[l].n > LSG_SMALL || 64 * rows > LSG_SMALL_SMEM) break;
-        lc = l;
-    }
-    size_t small_rows = 0;
-    for (int k = lc; k <= last; ++k) small_rows += (size_t)op.mg.lev[k].n;
-    const size_t small_smem = 64 * small_rows;
-    P.lc = lc;
-    P.levs = (LsgLevel *)(w + Lo.levs);
+    const int n1 = op.mgx.lev[lc + 1].n;   // the dense level
+    const size_t small_smem = 16 * ((size_t)lev[lc].n + 2 * mgx_stride(n1));
     P.B = B; P.X = X;
     P.V = (float *)(w + Lo.V); P.Z = (float *)(w + Lo.Z); P.w = (float *)(w + Lo.w);
     P.R = (double *)(w + Lo.R); P.rpart = (double *)(w + Lo.rpart); P.bpart = (double *)(w + Lo.bpart);
@@ -2423,22 +2306,12 @@ cudaError_t lsg_solve(const DevSolveOp &op, const double *B, double *X, int nv, 
     cudaError_t e;
     if ((e = cudaMemsetAsync(st, 0, sizeof(GmresStats), s)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(P.done, 0, sizeof(int), s)) != cudaSuccess) return e;
-    static std::once_flag smem_once;
-    static cudaError_t smem_err = cudaSuccess;
-    std::call_once(smem_once, [] {
-        smem_err = cudaFuncSetAttribute((const void *)k_mg_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)LSG_SMALL_SMEM);
-    });
-    if (smem_err != cudaSuccess) return smem_err;
-    if (small_smem > LSG_SMALL_SMEM) return cudaErrorInvalidValue;
     long long launches = 0;
     const dim3 rgrid((unsigned)Lo.nbx, (unsigned)((nv + LS_MG - 1) / LS_MG));
     const unsigned rblocks = resid_grid(W, (long long)rgrid.x * rgrid.y);
-    k_lsg_levels<<<1, 32, 0, s>>>(P);
     k_ls_sq<<<rgrid, 256, 0, s>>>(B, n, ld, nv, P.bpart);
-    launches += 2;
+    launches += 1;
     const unsigned gsmall = (unsigned)std::min(P.q4, 4 * sm_count());
-    const unsigned gn = lsg_blocks((long long)n * P.q4, lsg_grids().spmm);
     const dim3 red_grid((unsigned)Lo.RB, (unsigned)(nvp / 32));
     const unsigned tiles = lsg_blocks((long long)((n + 31) / 32) * (nvp / 32) * 256);
     P.maxc = lsg_maxc;
@@ -2462,29 +2335,24 @@ cudaError_t lsg_solve(const DevSolveOp &op, const double *B, double *X, int nv, 
             const float *src0 = j == 0 ? vj : P.w;
             float *vout0 = j == 0 ? nullptr : vj;
             float *zj = P.Z + (size_t)j * n * nvp;
+            auto src = [&](int l) -> const float * { return l == 0 ? src0 : lev[l].b; };
+            auto up = [&](int l) { return l == 0 ? zj : lev[l].x; };
             for (int l = 0; l < lc; ++l) {
-                k_mg_down<<<lsg_blocks((long long)P.lev[l].n * P.q4, lsg_grids().down), 256, 0, s>>>(
-                    P, P.lev[l], l == 0 ? src0 : P.lev[l].b, l == 0 ? vout0 : nullptr, j);
-                if (l + 1 < lc)
-                    k_mg_restrict<<<lsg_blocks((long long)P.lev[l + 1].n * P.q4), 256, 0, s>>>(P, P.lev[l], P.lev[l + 1], j);
-                launches += l + 1 < lc ? 2 : 1;
+                const int nc = op.mgx.lev[l + 1].n;
+                k_lsg_q<<<lsg_blocks((long long)nc * P.q4), 256, 0, s>>>(
+                    P, lev[l], nc, src(l), l == 0 && vout0, lev[l + 1].b, j);
             }
-            k_mg_small<<<gsmall, MG_SMALL_TB, small_smem, s>>>(P, src0, lc == 0 ? vout0 : nullptr, lc == 0 ? zj : P.lev[lc].x, j);
-            ++launches;
-            for (int l = lc - 1; l >= 0; --l) {
-                const float *xc = (l + 1 == lc) ? P.lev[lc].x : P.lev[l + 1].xo;
-                k_mg_prolong<<<lsg_blocks((long long)P.lev[l].n * P.q4), 256, 0, s>>>(P, P.lev[l], xc, j);
-                float *out = l == 0 ? zj : P.lev[l].xo;
-                k_mg_smooth<<<lsg_blocks((long long)P.lev[l].n * P.q4, lsg_grids().smooth), 256, 0, s>>>(
-                    P, P.lev[l], l == 0 ? vj : P.lev[l].b, out, j);
-                launches += 2;
-            }
-            k_lsg_spmm<<<gn, 256, 0, s>>>(P, j);
-            k_lsg_dot<<<red_grid, 256, 0, s>>>(P, j);
+            k_lsg_small<<<gsmall, MG_SMALL_TB, small_smem, s>>>(P, lev[lc], n1, (const float *)op.mgx.B[lc + 1],
+                                                               src(lc), lc == 0 ? vout0 : nullptr, up(lc), j);
+            for (int l = lc - 1; l >= 0; --l)
+                k_lsg_up<<<lsg_blocks((long long)lev[l].n * P.q4), 256, 0, s>>>(
+                    P, lev[l], src(l), l == 0 ? vout0 : nullptr, up(l + 1), up(l), j);
+            launches += 2 * lc + 1;
+            k_lsg_spmm_dot<<<red_grid, 256, 0, s>>>(P, j);
             k_lsg_hsum<<<(unsigned)((nv * (j + 1) + NWARP - 1) / NWARP), 256, 0, s>>>(P, j);
             k_lsg_update<<<red_grid, 256, 0, s>>>(P, j);
             k_lsg_givens<<<(unsigned)((nv + NWARP - 1) / NWARP), 256, 0, s>>>(P, j);
-            launches += 5;
+            launches += 4;
         }
         k_lsg_solve<<<lsg_blocks(nvp), 256, 0, s>>>(P);
         k_lsg_correct<<<tiles, 256, 0, s>>>(P);
@@ -2549,15 +2417,18 @@ SolvePath choose_path(const DevSolveOp &op, int nv, int m, Precision prec, bool 
     if (getenv("PHG_CHEB_LOCKSTEP") && !env_int("PHG_CHEB_LOCKSTEP", 1)) sh.path = 0;
     if (sh_out) *sh_out = sh;
     if (no_alloc) return SolvePath::Persistent;
-    // Level 5, mixed: 100 Laplace solves 2.7 ms persistent, 3.6 ms lockstep;
-    // 256 of them 7.4 and 5.5 ms.  Level 6: 37 of them 4.2 and 6.0 ms, 64 of
-    // them 8.4 and 6.1 ms.
+    // Level 5, mixed: 100 Laplace solves 2.7 ms persistent, 2.6 ms lockstep;
+    // 128 of them 3.7 and 2.7 ms, 256 of them 7.1 and 3.5 ms, 64 of them 1.7
+    // and 2.2 ms.  Level 6: 24 of them 2.4 and 3.7 ms, 32 of them 4.2 and 3.7
+    // ms, 48 of them 5.8 and 4.6 ms, but a time step of 32 members, whose solves
+    // start warm, 16.9 and 18.1 ms.
     const long long work = (long long)op.A.n * nv;
     if (uses_cheb(op, m)) {
         const bool ls = sh.path == 1 ? nv >= LS_MIN_TUNED : (sh.path == 0 ? false : work >= LS_MIN_WORK && nv >= 32);
         return prec == PREC_MIXED && ls ? SolvePath::ChebLockstep : SolvePath::Persistent;
     }
-    if (lsg_applicable(op, nv, prec, m) && (sh.path == 1 || (sh.path == -1 && work >= LSG_MIN_WORK)))
+    const long long least = lsg_cycles(op.A.n) > 3 ? LSG_MIN_WORK_L6 : LSG_MIN_WORK;
+    if (lsg_applicable(op, nv, prec, m) && (sh.path == 1 || (sh.path == -1 && work >= least && nv >= LSG_MIN_NV)))
         return SolvePath::MgLockstep;
     return SolvePath::Persistent;
 }
@@ -2923,7 +2794,6 @@ cudaError_t gmres_solve_multi(const DevSolveOp *const *ops, const int *nvk, cons
 
 void lockstep_prepare() {
     (void)ls_grids();
-    (void)lsg_grids();
 }
 
 }  // namespace phg

@@ -96,3 +96,33 @@ def test_ensemble_steps_graph_replayed(tmp_path):
     bv.run(b, 3)
     assert np.array_equal(a, b)
     assert bv.last_stats()["worst_relres"] <= 1e-10
+
+
+@pytest.mark.parametrize("level,nv,forced", [(3, 40, True), (4, 70, True), (5, 110, False), (6, 40, False)])
+def test_lockstep_solves_match_a_direct_solve(tmp_path, level, nv, forced):
+    """Levels where the small-level kernel starts at the finest level, one, two and three below it; ragged last
+    slices of 32; and, unforced, sizes just above the rule that chooses the path.  Against scipy's LU: the discrete
+    solution up to (condition number, about 1e3) x (relative residual, 1e-12), so 1e-9 as for every solve here."""
+    sp = pytest.importorskip("scipy.sparse")
+    from scipy.sparse.linalg import splu
+    m = phelm.Mesh.sphere(level)
+    lat, lon = m.latlon()
+    F = serve.solve_inputs(lat, lon, nv, seed=7)
+    bnd = np.random.default_rng(8).standard_normal((nv, m.outer_size))
+
+    def mat(name, cols):
+        ptr, col, val = m.csr(name)
+        return sp.csr_matrix((val, col, ptr), shape=(m.inner_size, cols))
+
+    inner = m.maps()["inner"]
+    want = splu(mat("lapl", m.inner_size).tocsc()).solve(
+        mat("idt", m.inner_size) @ F[:, inner].T + mat("bnd2", m.outer_size) @ bnd.T).T
+    ops = phelm.Operators(m, phelm.PHG_MIXED, tol=1e-12)
+    if forced:
+        force_path(tmp_path, m.inner_size, nv, 1)
+    k0 = phelm.kernel_launches()
+    got = phelm.SphereLaplace(ops).solve_batch(F, bnd)
+    assert phelm.kernel_launches() - k0 > 100      # the lockstep launches ran
+    assert ops.last_solve()["relres"] <= 1e-12
+    for k in range(nv):
+        assert rel(got[k][inner], want[k]) <= TOL, k

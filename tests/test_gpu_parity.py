@@ -208,15 +208,17 @@ def test_interleaved_apply_of_long_rows_equals_the_short_rows_product(level, nv,
     torch = pytest.importorskip("torch")
     m = phelm.Mesh.sphere(level)
     ops = phelm.Operators(m, phelm.PHG_MIXED, tol=1e-12)
-    n = m.inner_size
-    x = torch.randn((n, nv), generator=torch.Generator(device="cuda").manual_seed(level), device="cuda")
-    if special:
-        x[n // 3, 5], x[n - 1, nv - 1], x[0, 0], x[n // 2, nv // 2] = float("inf"), float("-inf"), float("nan"), 3e38
-    y, z = torch.full_like(x, 7.0), torch.empty((n, 16), device="cuda")
-    for name in ("lapl", "idt"):
-        ops.mult32(name, x, y)
-        for k in range(0, nv, 16):
-            ops.mult32(name, x[:, k:k + 16].contiguous(), z)
-            assert torch.equal(torch.nan_to_num(y[:, k:k + 16], 1.25, 2e38, -2e38),
-                               torch.nan_to_num(z, 1.25, 2e38, -2e38))
-            assert torch.equal(torch.isnan(y[:, k:k + 16]), torch.isnan(z))
+    n, st = m.inner_size, torch.cuda.Stream()
+    with torch.cuda.stream(st):   # everything in one stream's order
+        x = torch.randn((n, nv), generator=torch.Generator(device="cuda").manual_seed(level), device="cuda")
+        if special:
+            x[n // 3, 5], x[n - 1, nv - 1], x[0, 0], x[n // 2, nv // 2] = float("inf"), float("-inf"), float("nan"), 3e38
+        y, z = torch.full_like(x, 7.0), torch.empty((n, 16), device="cuda")
+        for name in ("lapl", "idt"):
+            ops.mult32(name, x, y, stream=st)
+            for k in range(0, nv, 16):
+                part = x[:, k:k + 16].contiguous()
+                ops.mult32(name, part, z, stream=st)
+                assert torch.equal(torch.nan_to_num(y[:, k:k + 16], 1.25, 2e38, -2e38),
+                                   torch.nan_to_num(z, 1.25, 2e38, -2e38))
+                assert torch.equal(torch.isnan(y[:, k:k + 16]), torch.isnan(z))
