@@ -227,8 +227,8 @@ def run_ours(args, ws, rank, local):
         barrier()
         wall = time.perf_counter() - t0
         launches = phelm.kernel_launches() - k0 - 0
-        prof = ops.profile_read(2)          # the Laplacian solves: gmres_kernel (the dominant kernel)
-        prof_all = ops.profile_read()       # every solver launch (gmres_kernel + cheb_kernel)
+        prof = ops.profile_read(2)          # the Laplacian solves: mgs_kernel (the dominant kernel)
+        prof_all = ops.profile_read()       # every solver launch (mgs_kernel + chs_kernel)
         ops.profile(False)
         dev_ms = sum(s.elapsed_time(e) for s, e in zip(starts, ends))
         st = bv.last_stats()
@@ -392,7 +392,7 @@ def run_ours(args, ws, rank, local):
     peak = peaks.get("hbm_gbs", 6800.0)
     achieved = prof["bytes"] / (prof["ms"] * 1e-3) / 1e9 if prof["ms"] > 0 else 0.0
     traffic = None
-    tf = os.path.join(HERE, "profiles", "gmres_traffic.json")
+    tf = os.path.join(HERE, "profiles", "mgs_traffic.json")
     if os.path.exists(tf):
         try:
             traffic = json.load(open(tf)).get("bytes_per_launch")
@@ -413,7 +413,7 @@ def run_ours(args, ws, rank, local):
     def r3(x):
         return None if x is None else float(f"{x:.4g}")
 
-    roof = {"kernel": "gmres_kernel<float>", "bound": "hbm", "achieved": r3(achieved), "peak": peak, "unit": "GB/s",
+    roof = {"kernel": "mgs_kernel<float>", "bound": "hbm", "achieved": r3(achieved), "peak": peak, "unit": "GB/s",
             "frac": r3(achieved / peak), "traffic": traffic,
             "bytes_per_launch": r3(prof["bytes"] / max(prof["launches"], 1)),
             "ms_per_launch": r3(prof["ms"] / max(prof["launches"], 1)),

@@ -6,7 +6,8 @@
 //     d <- ca d + cb D^-1 (r - A e),  e <- e + d
 // on r / ||r|| in the Krylov precision and adds ||r|| e to x.  A step is one
 // gather of seven neighbours a row, so a single right-hand side is bound by
-// the hand-over between steps and many by the FP64 (or gather) rate:
+// the hand-over between steps and many by the FP64 (or gather) rate (against
+// cheb_kernel, level 6 FP64: one 222 -> 90 us, the Jacobian's eight 554 -> 281):
 //
 //  * the iterate lives in stamped cells (phg_stamp.cuh): a row takes step k as
 //    soon as its neighbours' step k - 1 is there, no barrier within a cycle;

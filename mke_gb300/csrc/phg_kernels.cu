@@ -79,7 +79,7 @@ __global__ void k_apply(DevEll A, DevCols C, const double *xin, int ldx, const i
 // Bound by the FP64 pipe for many members (112 separate multiplies and adds per
 // row and member) and by latency for one: half a row per thread (the four
 // products of one field), all its gathers issued together (level 6, one
-// member: 25.4 -> 13.7 us).
+// member: 24.5 -> 21.2 us under the profiler; 14.6 of FP64 issue).
 __global__ void __launch_bounds__(TB) k_jac_rhs(JacOps J, const double *u, const double *w, int ld, const int *imap,
                                                 const int *bmap, double *out, int ldo, int nv) {
     const int n = J.d1.n, W = J.d1.W;
