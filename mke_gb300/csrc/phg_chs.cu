@@ -386,13 +386,25 @@ size_t chs_work_bytes(const DevSolveOp &op, int nv, Precision prec, int sms) {
     return al(per * (prec == PREC_MIXED ? 8 : 16)) + al(per * (prec == PREC_MIXED ? 4 : 8));
 }
 
+cudaError_t chs_prepare() {
+    int lim;
+    cudaError_t e = cudaSuccess;
+    for (Precision prec : {PREC_FP64, PREC_MIXED})
+        for (int C : {1, 2, 4, 8})
+            for (bool one : {false, true})
+                if (e == cudaSuccess) e = chs_smem_limit(prec, C, one, &lim);
+    return e;
+}
+
 cudaError_t chs_solve(const DevSolveOp &op, const ChsArgs &q, cudaStream_t s) {
     const int n = op.A.n, C = chunk_of(n, q.nv, q.prec, q.sms), chunks = (q.nv + C - 1) / C;
     const size_t es = q.prec == PREC_MIXED ? 4 : 8;
     const int sms = (q.max_sms > 0 && q.max_sms < q.sms) ? q.max_sms : q.sms;
-    // one block per SM, shared out over the chunks
-    const int groups = std::min(chunks, sms);
-    int G = sms / groups;
+    // one block per SM, shared out over the chunks; two smaller ones where the
+    // caller leaves this launch a part of the SMs (see mgs_solve)
+    const bool half = sms < q.sms;
+    const int slots = half ? 2 * sms : sms, groups = std::min(chunks, std::min(slots, q.sms));
+    int G = slots / groups;
     if (q.rpb > 0) G = std::min(G, (n + q.rpb - 1) / q.rpb);
     if (small_system(n, q.prec)) G = 1;
     G = std::max(G, 1);
@@ -400,6 +412,7 @@ cudaError_t chs_solve(const DevSolveOp &op, const ChsArgs &q, cudaStream_t s) {
     int limit = 0;
     cudaError_t e = chs_smem_limit(q.prec, C, one, &limit);
     if (e != cudaSuccess) return e;
+    if (half) limit = std::min(limit, 104 * 1024);
     ChsParams p;
     memset(&p, 0, sizeof p);
     const size_t rpb = (size_t)((n + G - 1) / G);
@@ -427,7 +440,7 @@ cudaError_t chs_solve(const DevSolveOp &op, const ChsArgs &q, cudaStream_t s) {
     memcpy(p.cb, q.plan->cb, sizeof p.cb);
     p.wait_limit = q.wait_limit;
     // threads for a row and right-hand side each, as far as there are
-    const int most = q.prec == PREC_MIXED ? 1024 : 768;
+    const int most = half ? 384 : q.prec == PREC_MIXED ? 1024 : 768;
     const int threads = (int)std::min<size_t>(most, std::max<size_t>(256, (rpb * C + 31) / 32 * 32));
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute coop[1];

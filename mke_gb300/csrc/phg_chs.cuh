@@ -34,6 +34,9 @@ struct ChsArgs {
 };
 
 size_t chs_work_bytes(const DevSolveOp &op, int nv, Precision prec, int sms);
+// load every instantiation (operator creation calls it): the first launch of a
+// kernel that is loaded then waits for the device, and so for other streams' work
+cudaError_t chs_prepare();
 cudaError_t chs_solve(const DevSolveOp &op, const ChsArgs &a, cudaStream_t s);
 
 }  // namespace phg

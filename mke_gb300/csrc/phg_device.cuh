@@ -189,7 +189,7 @@ int tune_load(const char *path);
 // launches over all right-hand sides (Chebyshev / multigrid FGMRES)
 enum class SolvePath { Persistent, ChebLockstep, MgLockstep };
 SolvePath choose_path(const DevSolveOp &op, int nv, int m, Precision prec, bool no_alloc, const SolveShape *shape,
-                      SolveShape *sh_out);
+                      SolveShape *sh_out, int max_sms = 0);
 // query the lockstep kernels' launch grids once; call outside any stream
 // capture (operator creation does) so that a captured solve only reads them
 void lockstep_prepare();

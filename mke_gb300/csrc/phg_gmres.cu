@@ -2409,7 +2409,7 @@ static cudaError_t allow_smem(Precision prec, bool multi = false) {
 // (given, else the tuned one; environment overrides) decides between the
 // persistent kernels and the lockstep launches.  sh_out: the shape used.
 SolvePath choose_path(const DevSolveOp &op, int nv, int m, Precision prec, bool no_alloc, const SolveShape *shape,
-                      SolveShape *sh_out) {
+                      SolveShape *sh_out, int max_sms) {
     SolveShape sh;
     if (shape) sh = *shape;
     else tune_get_solve(solve_family(op), op.A.n, prec, nv, &sh);
@@ -2422,7 +2422,12 @@ SolvePath choose_path(const DevSolveOp &op, int nv, int m, Precision prec, bool 
     // and 2.2 ms.  Level 6: 24 of them 2.4 and 3.7 ms, 32 of them 4.2 and 3.7
     // ms, 48 of them 5.8 and 4.6 ms, but a time step of 32 members, whose solves
     // start warm, 16.9 and 18.1 ms.
-    const long long work = (long long)op.A.n * nv;
+    // A capped caller's persistent kernels have their share of the SMs, its
+    // lockstep launches whatever is free: the products scale with the share (a
+    // serving trace of levels 3 to 7: 715 -> 755 requests/s).
+    const int sms = sm_count();
+    const long long work = (long long)op.A.n * nv * (max_sms > 0 && max_sms < sms ? sms : 1) /
+                           (max_sms > 0 && max_sms < sms ? max_sms : 1);
     if (uses_cheb(op, m)) {
         const bool ls = sh.path == 1 ? nv >= LS_MIN_TUNED : (sh.path == 0 ? false : work >= LS_MIN_WORK && nv >= 32);
         return prec == PREC_MIXED && ls ? SolvePath::ChebLockstep : SolvePath::Persistent;
@@ -2433,11 +2438,19 @@ SolvePath choose_path(const DevSolveOp &op, int nv, int m, Precision prec, bool 
     return SolvePath::Persistent;
 }
 
-// workspace of the path the solve will take (the lockstep multigrid path
-// needs only its own 2m + 1 interleaved vectors; the others the layout above)
+// workspace of a solve of nv right-hand sides, or fewer, on whichever path it takes
 size_t gmres_work_bytes(const DevSolveOp &op, int nv, int m, Precision p, const SolveShape *shape) {
-    if (choose_path(op, nv, m, p, false, shape, nullptr) == SolvePath::MgLockstep) return lsg_layout(op, nv, m).total;
-    return layout(op, nv, m, p).total;
+    const bool lock = choose_path(op, nv, m, p, false, shape, nullptr) == SolvePath::MgLockstep;
+    // Enough for fewer right-hand sides too, whose persistent solve may need more
+    // than the lockstep one of all: a buffer that grows between a server's turns
+    // waits for every stream.
+    const long long least = lsg_cycles(op.A.n) > 3 ? LSG_MIN_WORK_L6 : LSG_MIN_WORK;
+    const int few = (int)std::min<long long>(nv, std::max<long long>(LSG_MIN_NV - 1, (least - 1) / op.A.n));
+    size_t bytes = layout(op, lock ? few : nv, m, p).total;
+    // and a capped launch may take the lockstep path from fewer on
+    if (lock || choose_path(op, nv, m, p, false, shape, nullptr, 1) == SolvePath::MgLockstep)
+        bytes = std::max(bytes, lsg_layout(op, nv, m).total);
+    return bytes;
 }
 
 cudaError_t gmres_solve(const DevSolveOp &op, const double *B, double *X, int nv, int ld,
@@ -2450,7 +2463,7 @@ cudaError_t gmres_solve(const DevSolveOp &op, const double *B, double *X, int nv
     const size_t es = prec == PREC_MIXED ? 4 : 8;
     const bool cheb = uses_cheb(op, m);
     SolveShape sh;
-    const SolvePath path = choose_path(op, nv, m, prec, no_alloc, shape, &sh);
+    const SolvePath path = choose_path(op, nv, m, prec, no_alloc, shape, &sh, max_sms);
     const bool lockstep = path == SolvePath::ChebLockstep;
     // ensembles of the multigrid Laplacian in the mixed path: lockstep launches
     if (path == SolvePath::MgLockstep) {
@@ -2794,6 +2807,15 @@ cudaError_t gmres_solve_multi(const DevSolveOp *const *ops, const int *nvk, cons
 
 void lockstep_prepare() {
     (void)ls_grids();
+    // a kernel that fails to load says so again when a solve launches it
+    if (mgs_prepare() != cudaSuccess || chs_prepare() != cudaSuccess) cudaGetLastError();
+    cudaFuncAttributes fa;
+    for (const void *f : {(const void *)k_lsg_q, (const void *)k_lsg_small, (const void *)k_lsg_up,
+                          (const void *)k_lsg_spmm_dot, (const void *)k_lsg_hsum, (const void *)k_lsg_update,
+                          (const void *)k_lsg_givens, (const void *)k_lsg_begin, (const void *)k_lsg_zero,
+                          (const void *)k_lsg_v0, (const void *)k_lsg_solve, (const void *)k_lsg_correct,
+                          (const void *)k_ls_sq, (const void *)k_ls_nrm, (const void *)k_ls_scale})
+        if (cudaFuncGetAttributes(&fa, f) != cudaSuccess) cudaGetLastError();
 }
 
 }  // namespace phg

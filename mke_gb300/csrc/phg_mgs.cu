@@ -878,6 +878,14 @@ bool mgs_applicable(const DevSolveOp &op) {
     return op.mgx.nlev >= 2 && (op.block4 ? op.blk.c != nullptr : op.A.W <= 8);
 }
 
+cudaError_t mgs_prepare() {
+    int lim;
+    cudaError_t e = cudaSuccess;
+    for (Precision prec : {PREC_FP64, PREC_MIXED})
+        for (int kind = 0; kind < 3 && e == cudaSuccess; ++kind) e = mgs_smem_limit(prec, kind, &lim);
+    return e;
+}
+
 cudaError_t mgs_solve(const DevSolveOp &op, const MgsArgs &q, cudaStream_t s) {
     const MgxDev &x = op.mgx;
     const bool blk = op.block4 != 0;
@@ -892,9 +900,12 @@ cudaError_t mgs_solve(const DevSolveOp &op, const MgsArgs &q, cudaStream_t s) {
     // for three blocks each (level 5, 100 FP64 right-hand sides: 6.4 ms with one
     // block each on 100 of 152 SMs, 4.3 ms with three half-size blocks; level 4,
     // 152 mixed ones: 0.92 ms with one block, 1.20 ms with two halves).
-    const bool many = q.nv > sms || (2 * q.nv > sms && 2 * sms / q.nv >= 3);
-    int workers = many ? 256 : (mixed ? 768 : 512);
-    const int cap = many ? 2 * sms : sms;
+    // Two smaller blocks also where the caller leaves this launch a part of the
+    // SMs: others run beside it, and an SM seldom empties for a block that
+    // needs all of it.
+    const bool half = sms < q.sms || q.nv > sms || (2 * q.nv > sms && 2 * sms / q.nv >= 3);
+    int workers = half ? 256 : (mixed ? 768 : 512);
+    const int cap = half ? 2 * sms : sms;
     const int groups = std::min(q.nv, cap);
     int G = cap / groups;
     if (q.rpb > 0) G = std::min(G, (n + q.rpb - 1) / q.rpb);
@@ -904,7 +915,7 @@ cudaError_t mgs_solve(const DevSolveOp &op, const MgsArgs &q, cudaStream_t s) {
     cudaError_t e = mgs_smem_limit(q.prec, blk ? 2 : one ? 1 : 0, &limit);
     if (e != cudaSuccess) return e;
     size_t budget = (size_t)limit;
-    if (many) budget = std::min<size_t>(budget, 104 * 1024);
+    if (half) budget = std::min<size_t>(budget, 104 * 1024);
 
     MgsParams p;
     memset(&p, 0, sizeof p);
@@ -923,7 +934,7 @@ cudaError_t mgs_solve(const DevSolveOp &op, const MgsArgs &q, cudaStream_t s) {
             const bool cached = mgs_fixed_smem() + es * ent < 0.6 * (double)budget;
             const double rate = mixed ? (cached ? 48.0 : 14.0) : (cached ? 1.6 : 1.5);
             const int hand = (k > 0 ? k : 0) + (top > 0 ? top : 0);
-            const double cost = hand * (one ? 150.0 : 1500.0) + ent / rate * (many ? 2.0 : 1.0);
+            const double cost = hand * (one ? 150.0 : 1500.0) + ent / rate * (half ? 2.0 : 1.0);
             if (cost < best) { best = cost; p.top = top; p.bot = k; }
         }
     // shared memory: the coarse levels' rows, the dense rows, then the finest

@@ -23,6 +23,9 @@ struct MgsArgs {
 
 bool mgs_applicable(const DevSolveOp &op);
 size_t mgs_scratch_bytes(const DevSolveOp &op, Precision prec);   // per right-hand side in flight
+// load every instantiation (operator creation calls it): the first launch of a
+// kernel that is loaded then waits for the device, and so for other streams' work
+cudaError_t mgs_prepare();
 cudaError_t mgs_solve(const DevSolveOp &op, const MgsArgs &a, cudaStream_t s);
 
 }  // namespace phg

@@ -126,3 +126,22 @@ def test_lockstep_solves_match_a_direct_solve(tmp_path, level, nv, forced):
     assert ops.last_solve()["relres"] <= 1e-12
     for k in range(nv):
         assert rel(got[k][inner], want[k]) <= TOL, k
+
+
+@pytest.mark.parametrize("level,nv,sms", [(4, 40, 8), (5, 20, 16), (5, 40, 100)])
+def test_capped_launches_match_uncapped_ones(level, nv, sms):
+    """A caller that leaves these solves a part of the SMs gets half-size blocks, and from fewer right-hand sides the
+    lockstep launches, in a workspace that the first, uncapped call already sized; every solve runs to 1e-12."""
+    m = phelm.Mesh.sphere(level)
+    lat, lon = m.latlon()
+    F = serve.solve_inputs(lat, lon, nv, seed=3)
+    ops = phelm.Operators(m, phelm.PHG_MIXED, tol=1e-12)
+    L = phelm.SphereLaplace(ops)
+    want = L.solve_batch(F)
+    held = phelm.device_bytes() if hasattr(phelm, "device_bytes") else None
+    ops.set_sms(sms)
+    got, few = L.solve_batch(F), L.solve_batch(F[:3])
+    assert ops.last_solve()["relres"] <= 1e-12
+    if held is not None:
+        assert phelm.device_bytes() == held
+    assert rel(got, want) <= TOL and rel(few, want[:3]) <= TOL
