@@ -2239,13 +2239,24 @@ int lin_calc1(phg_barvortex_s *b, double *out, const double *F, const double *bn
     return PHG_OK;
 }
 
-// full vector out = SphereLaplace::solve(F, bnd)
-int lin_lsolve(phg_barvortex_s *b, double *out, const double *F, const double *bnd, int &slot, cudaStream_t s) {
+// The operator as gmres_kernel and cheb_kernel take it, without the tables of
+// the stamped-cell solvers
+DevSolveOp barrier_op(const DevSolveOp &op) {
+    DevSolveOp g = op;
+    g.mgx = MgxDev();
+    g.c7 = nullptr;
+    g.v7 = nullptr;
+    return g;
+}
+
+// full vector out = SphereLaplace::solve(F, bnd), by L
+int lin_lsolve(phg_barvortex_s *b, double *out, const double *F, const DevSolveOp &L, const double *bnd, int &slot,
+               cudaStream_t s) {
     phg_ops_s *o = b->o;
     double *rp = b->lrp.as<double>(), *x = b->lx.as<double>();
     CK(apply_op(o->ML.op.A, o->bnd2.c, F, o->V, o->imap(), bnd, o->os, nullptr, rp, o->rs, 1, s));
     CK(cudaMemsetAsync(x, 0, 8 * (size_t)o->rs, s));
-    int r = solve(o, o->L.op, rp, x, 1, o->rs, o->tol, slot++, s);
+    int r = solve(o, L, rp, x, 1, o->rs, o->tol, slot++, s);
     if (r) return r;
     CK(p2u(out, o->V, x, o->rs, bnd, o->os, o->p2io.as<int>(), o->isb.as<int>(), o->V, 1, s));
     return PHG_OK;
@@ -2310,6 +2321,15 @@ int lin_backward(phg_barvortex_s *b) {
     return PHG_OK;
 }
 
+// Above this many rows (level 6 on) a mixed-precision adjoint keeps the
+// group-barrier solvers.  The Laplacians after its solves amplify what the
+// stopping test (1e-12) leaves of the residual, noise at the grid scale, to
+// 0.5..1.6e-9 of the result at level 6 and 2..4.5e-9 at level 7, so solvers
+// that round in another order give another result within that: 2.0e-9 and
+// 5.7e-9 away (level 5: 3.6e-10), where these give the same to 4e-16.  It
+// costs 1.52 -> 3.55 ms at level 6, 3.5 -> 7.8 ms at level 7.
+constexpr int ADJ_KEEP_ROWS = 20000;
+
 // kind 0: calc_L, 1: calc_L_1 (adds into u1), 2: calc_LT; device pointers
 int lin_dev(phg_barvortex_s *b, int kind, double *u1, const double *u, const double *z, const double *bnd_u,
             const double *bnd_w, cudaStream_t s) {
@@ -2350,13 +2370,15 @@ int lin_dev(phg_barvortex_s *b, int kind, double *u1, const double *u, const dou
         const DevSolveOp &M = kind == 0 ? b->A.op : b->Aback.op;
         const DevCols &Bc = kind == 0 ? b->Ab.c : b->Abackb.c;
         if ((r = lin_msolve(b, u1, u1, M, Bc, bnd_w, slot, s))) return r;
-        if ((r = lin_lsolve(b, u1, u1, bnd_u, slot, s))) return r;
+        if ((r = lin_lsolve(b, u1, u1, o->L.op, bnd_u, slot, s))) return r;
     } else {
         // examples/barvortex_impl.h:485-535
         CK(cudaMemcpyAsync(in, z, 8 * NV, cudaMemcpyDeviceToDevice, s));   // v1 may alias z
         if ((r = lin_calc1(b, zl, in, bnd_w, slot, s))) return r;
-        if ((r = lin_lsolve(b, u1, u, bnd_u, slot, s))) return r;
-        if ((r = lin_msolve(b, u1, u1, b->A.op, b->Ab.c, bnd_w, slot, s))) return r;
+        const bool keep = o->prec == PHG_MIXED && o->rs > ADJ_KEEP_ROWS;
+        const DevSolveOp Lg = keep ? barrier_op(o->L.op) : o->L.op, Ag = keep ? barrier_op(b->A.op) : b->A.op;
+        if ((r = lin_lsolve(b, u1, u, Lg, bnd_u, slot, s))) return r;
+        if ((r = lin_msolve(b, u1, u1, Ag, b->Ab.c, bnd_w, slot, s))) return r;
         if ((r = lin_calc1(b, pt1, u1, bnd_w, slot, s))) return r;
         CK(axpbz(pt1, pt1, 1.0 / tau - (1.0 - th) * sg, pt1, 0.0, NV, s));
         if ((r = lin_calc1(b, pt2, u1, bnd_w, slot, s))) return r;
