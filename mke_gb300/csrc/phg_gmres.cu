@@ -59,8 +59,8 @@ constexpr int LS_MIN_TUNED = 8;  // the fewest right-hand sides for which the au
 // block, the former win once the vectors outgrow that -- by rows x right-hand
 // sides, from about these products on (measured; see choose_path)
 constexpr long long LS_MIN_WORK = 8000000;    // Chebyshev solves
-// multigrid Laplacians (above level 5 the lockstep path runs a cycle more), and
-// the fewest right-hand sides
+// multigrid Laplacians (above level 5 one right-hand side's persistent solve fills
+// the chip sooner), and the fewest right-hand sides
 constexpr long long LSG_MIN_WORK = 1100000, LSG_MIN_WORK_L6 = 1500000;
 constexpr int LSG_MIN_NV = 16;
 
@@ -1728,11 +1728,18 @@ int env_int(const char *name, int dflt) {
 // index range with a grid-stride loop over a grid capped at a few blocks per
 // SM, so a launch that finds its flag set costs little.
 constexpr int LSG_M = 8;        // Arnoldi steps per refinement cycle
-// refinement cycles at most: three of eight steps reach 1e-12 from a zero start
-// up to level 5 and stop at 1e-11 on level 6, where a fourth takes all right-hand
-// sides there; below it would only add skipped launches (level 5 x 256 solves
-// 3.4 -> 4.0 ms)
-inline int lsg_cycles(int n) { return n > 20000 ? 4 : 3; }
+// Refinement cycles at most.  Right-hand sides of all kinds (noise, single
+// points, high degrees, a constant) reach 1e-12 from a zero start within four
+// cycles of eight steps on levels 3, 4, 6 and 7, as far as the persistent kernel
+// reaches it at all (level 8: 1.2e-12).  On level 5 three leave a constant at
+// 4.9e-12 (the persistent kernel 2.6e-12, after 33 steps), and a fourth only adds
+// skipped launches to the others (256 solves 3.4 -> 4.0 ms; the fourth on level
+// 4 costs 500 solves 2.39 -> 2.65 ms).  A tighter tolerance takes a cycle more.
+inline int lsg_cycles(int n, double tol) {
+    return (n > 10000 && n <= 20000 ? 3 : 4) + (tol < 1e-12 ? 1 : 0);
+}
+// rows x right-hand sides from which the path is taken
+inline long long lsg_least(int n) { return n > 20000 ? LSG_MIN_WORK_L6 : LSG_MIN_WORK; }
 constexpr int LSG_MINRHS = 8;   // fewest right-hand sides the path accepts
 constexpr int LSG_SMALL = 700;  // levels of at most this many rows run in one shared-memory kernel
 
@@ -2256,7 +2263,8 @@ int lsg_small_level(const MgxDev &x) {
 }
 
 bool lsg_applicable(const DevSolveOp &op, int nv, Precision p, int restart) {
-    if (p != PREC_MIXED || !op.mgd || op.block4 || op.A.W > 8 || !op.a32 || nv < LSG_MINRHS || restart < 2) return false;
+    // (a restart below a cycle's eight steps: the cycles would end before the tolerance; the persistent kernel goes on)
+    if (p != PREC_MIXED || !op.mgd || op.block4 || op.A.W > 8 || !op.a32 || nv < LSG_MINRHS || restart < LSG_M) return false;
     const int lc = lsg_small_level(op.mgx);
     if (lc < 0 || !op.mgx.B[lc + 1]) return false;
     return (long long)op.A.n * ((nv + 31) / 32 * 8) < (1LL << 31);
@@ -2268,7 +2276,7 @@ unsigned lsg_blocks(long long work) {
 
 cudaError_t lsg_solve(const DevSolveOp &op, const double *B, double *X, int nv, int ld, int restart, int max_iter,
                       double tol, double inner_rtol, char *w, GmresStats *st, double mg_row_bytes, cudaStream_t s) {
-    const int lsg_maxc = lsg_cycles(op.A.n);
+    const int lsg_maxc = lsg_cycles(op.A.n, tol);
     const LsgLayout Lo = lsg_layout(op, nv, restart);
     const int n = op.A.n, W = op.A.W, nvp = Lo.nvp, m = Lo.m, lc = lsg_small_level(op.mgx);
     LsgParams P;
@@ -2432,8 +2440,8 @@ SolvePath choose_path(const DevSolveOp &op, int nv, int m, Precision prec, bool 
         const bool ls = sh.path == 1 ? nv >= LS_MIN_TUNED : (sh.path == 0 ? false : work >= LS_MIN_WORK && nv >= 32);
         return prec == PREC_MIXED && ls ? SolvePath::ChebLockstep : SolvePath::Persistent;
     }
-    const long long least = lsg_cycles(op.A.n) > 3 ? LSG_MIN_WORK_L6 : LSG_MIN_WORK;
-    if (lsg_applicable(op, nv, prec, m) && (sh.path == 1 || (sh.path == -1 && work >= least && nv >= LSG_MIN_NV)))
+    if (lsg_applicable(op, nv, prec, m) &&
+        (sh.path == 1 || (sh.path == -1 && work >= lsg_least(op.A.n) && nv >= LSG_MIN_NV)))
         return SolvePath::MgLockstep;
     return SolvePath::Persistent;
 }
@@ -2444,8 +2452,7 @@ size_t gmres_work_bytes(const DevSolveOp &op, int nv, int m, Precision p, const 
     // Enough for fewer right-hand sides too, whose persistent solve may need more
     // than the lockstep one of all: a buffer that grows between a server's turns
     // waits for every stream.
-    const long long least = lsg_cycles(op.A.n) > 3 ? LSG_MIN_WORK_L6 : LSG_MIN_WORK;
-    const int few = (int)std::min<long long>(nv, std::max<long long>(LSG_MIN_NV - 1, (least - 1) / op.A.n));
+    const int few = (int)std::min<long long>(nv, std::max<long long>(LSG_MIN_NV - 1, (lsg_least(op.A.n) - 1) / op.A.n));
     size_t bytes = layout(op, lock ? few : nv, m, p).total;
     // and a capped launch may take the lockstep path from fewer on
     if (lock || choose_path(op, nv, m, p, false, shape, nullptr, 1) == SolvePath::MgLockstep)
