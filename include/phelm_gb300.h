@@ -132,11 +132,12 @@ int phg_ops_set_solver(phg_ops o, int restart, double tol, int max_iter);
  * at the same time on different streams then share the GPU instead of
  * queueing behind each other.  No reference counterpart. */
 int phg_ops_set_sms(phg_ops o, int max_sms);
-/* Bounded waits (no reference counterpart): a group-barrier wait inside the
- * persistent solver kernels of this handle gives up after `cycles` GPU clock
- * cycles (0 = the default, about one second); the launch then ends early and
- * the call (or the next phg_ops_check) returns PHG_ERR_TIMEOUT.  The handle
- * stays usable. */
+/* Bounded waits (no reference counterpart): a wait inside the persistent
+ * solver kernels of this handle, at a group barrier or for another block's
+ * value, gives up after `cycles` GPU clock cycles (0 = the default, about one
+ * second; a wait for a value looks at the clock at every 64th load).  Its
+ * group stops with it, the launch ends early and the call (or the next
+ * phg_ops_check) returns PHG_ERR_TIMEOUT.  The handle stays usable. */
 int phg_ops_set_wait_limit(phg_ops o, long long cycles);
 /* Statistics of the last solve on this handle (host memory). */
 int phg_ops_last_solve(phg_ops o, int *iters, int *cycles, double *relres);

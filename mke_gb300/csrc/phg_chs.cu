@@ -69,6 +69,7 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 1024 : 768, 1) chs_kernel(co
     VT *cf = (VT *)(red + 2 * C * RSC);                 // ca, cb in the Krylov precision
     __shared__ double s_sum[2 * C], s_bn[C], s_bi[C], s_beta[C], s_prev[C], s_scale[C], s_rel[C];
     __shared__ int s_open[C], s_stat[C], s_iter[C], s_cyc[C], s_kc, s_dead;
+    __shared__ long long s_since[32];
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, NT = blockDim.x, NW = NT >> 5;
     const int n = p.n, G = p.G, W = p.W, nv = p.nv;
@@ -87,7 +88,7 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 1024 : 768, 1) chs_kernel(co
     }
     unsigned *bar = p.bar + 2 * grp;
     int *err = p.err;
-    const Waits wt = {err, (unsigned long long *)bar, &s_dead, wait_rounds(p.wait_limit)};
+    const Waits wt = {err, (unsigned long long *)bar, &s_dead, s_since, p.wait_limit};
     double *part2 = p.part + (size_t)(blockIdx.x - bi) * 2 * (MAXM + 2);
     int parity = 0;
     int r0, r1;

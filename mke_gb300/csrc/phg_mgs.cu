@@ -191,6 +191,7 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
     __shared__ double scal[5], s_a, s_target;
     __shared__ VT s_inv;
     __shared__ int s_stop, s_dead, s_go, s_zero;
+    __shared__ long long s_since[32];
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int NW = (blockDim.x >> 5) - 1;    // worker warps; the last warp is the helper
@@ -202,7 +203,7 @@ __global__ void __launch_bounds__(sizeof(VT) == 4 ? 800 : 544, 1) mgs_kernel(con
     if (grp >= p.groups) return;
     unsigned *bar = p.bar + 2 * grp;
     int *err = p.err;
-    const Waits wt = {err, (unsigned long long *)bar, &s_dead, wait_rounds(p.wait_limit)};
+    const Waits wt = {err, (unsigned long long *)bar, &s_dead, s_since, p.wait_limit};
     if (threadIdx.x == 0) {
         wait_limit_slot() = p.wait_limit;
         bar_epoch() = 0;

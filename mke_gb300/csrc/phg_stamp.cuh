@@ -16,9 +16,12 @@
 //
 // The lanes of a warp read together and go on together (a loop per lane would
 // let lanes that wait block lanes that have to write).  Every wait is bounded: a
-// warp that repeats a load for about the launch's wait limit raises the launch's error
-// flag, poisons its group's barrier word and marks its block, whose other
-// warps stop waiting too and whose next __syncthreads leads out of the kernel.
+// warp looks at the clock at every 64th load, and once it has waited for the
+// launch's limit (beyond the first 64 loads) it raises the launch's error flag.
+// A warp that gives up, for its own limit or for the flag, poisons its group's
+// barrier word, so that no block of the group waits there for its block, and
+// marks its block, whose other warps stop waiting too and whose next
+// __syncthreads leads out of the kernel.
 #pragma once
 #include "phg_group.cuh"
 
@@ -61,11 +64,9 @@ struct Waits {
     int *err;                   // the launch's error flag (the status of its record)
     unsigned long long *bar;    // the group's barrier word
     int *dead;                  // shared: this block gives up
-    unsigned rounds;            // loads a wait may repeat: the wait limit at about 400 cycles (a trip to L2) each
+    long long *since;           // shared, one per warp: when its wait began (a register would be held through every wait)
+    long long limit;            // clock cycles that a wait may take
 };
-__device__ __forceinline__ unsigned wait_rounds(long long limit) {
-    return (unsigned)min(max(limit / 400, 64LL), 1LL << 31);
-}
 
 // x[q] = the value of cell p[c[q]] once all N of every lane carry `stamp`.
 // All 32 lanes call it together.
@@ -81,12 +82,12 @@ __device__ __forceinline__ void wait_cells(VT (&x)[N], const Cell<VT> *p, const 
         for (int q = 0; q < N; ++q) miss |= e[q] ^ stamp;
         if (!__any_sync(0xffffffffu, miss != 0)) return;
         if ((round & 63u) == 63u) {   // inline: a call here would put a register save at every wait
-            const bool late = round >= w.rounds;
+            volatile long long *since = w.since + (threadIdx.x >> 5);
+            if (round == 63u) *since = clock64();
+            const bool late = clock64() - *since > w.limit;
             if (__any_sync(0xffffffffu, late || *(volatile int *)w.dead || *(volatile int *)w.err == STATUS_TIMEOUT)) {
-                if (late) {
-                    atomicMax(w.err, STATUS_TIMEOUT);
-                    atomicOr(w.bar, BAR_POISON);
-                }
+                if (late) atomicMax(w.err, STATUS_TIMEOUT);
+                atomicOr(w.bar, BAR_POISON);
                 *(volatile int *)w.dead = 1;
                 return;
             }
