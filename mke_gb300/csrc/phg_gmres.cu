@@ -2641,8 +2641,8 @@ cudaError_t gmres_solve(const DevSolveOp &op, const double *B, double *X, int nv
         cudaStreamSynchronize(s);
         static const char *nm[T_NPHASE] = {"resid", "vcycle", "spmv_dot", "dot_sum", "update", "norm_sum",
                                            "givens", "corr", "barrier_wait", "barriers", "total"};
-        fprintf(stderr, "[phases] n=%d nv=%d groups=%d G=%d mg=%d iters=%d cycles=%d |", n, nv, groups, G,
-                op.mgd ? op.mg.nlev : 0, st.iters, st.cycles);
+        fprintf(stderr, "[phases] n=%d nv=%d groups=%d G=%d mg=%d cluster=%d iters=%d cycles=%d |", n, nv, groups, G,
+                op.mgd ? op.mg.nlev : 0, CS, st.iters, st.cycles);
         for (int k = 0; k < T_NPHASE; ++k) fprintf(stderr, " %s=%lld", nm[k], k == T_BARRIERS ? h[k] : h[k] / 1000);
         fprintf(stderr, " (kcycles)\n");
     }
