@@ -2536,6 +2536,7 @@ int build_bc_blk(phg_ops_s *o, const Csr &A, const std::vector<double> &dinv, do
     if (!plan) return PHG_OK;
     const int rs = o->rs;
     const Csr &M = o->mesh->ops.idt;
+    if (!block_parts_complete(A, M, o->mesh->ops.lapl)) return PHG_OK;   // the level-by-level solver takes any
     // the blocks' entries on the mass matrix's pattern
     auto block = [&](int br, int bc) {
         Csr B = M;

@@ -118,6 +118,11 @@ struct MgPlan {
 };
 Csr csr_multiply(const Csr &A, const Csr &B);   // columns ascending
 bool build_mg_plan(const Csr &fine, const MgHierarchy &h, double omega, MgPlan &p);
+// Whether a block system in block order (w1, w2, u1, u2) consists of the parts
+// that the composed block solver applies and of nothing else: entries on M's
+// pattern in the w rows' w columns and the w2 rows' u2 columns, M in a u row's
+// own layer's w columns and -L in its own columns.
+bool block_parts_complete(const Csr &A, const Csr &M, const Csr &L);
 // BarVortex forward matrix c1 * mass + c2 * slaplace (examples/barvortex_impl.h:57-78)
 void assemble_barvortex(const Mesh &m, double c1, double c2, Csr &A, Csr &Abnd);
 // Baroclin 4rs x 4rs block matrix (examples/baroclin.cpp:119-180) and the

@@ -78,6 +78,43 @@ std::vector<double> multiply(const Csr &A, const std::vector<double> &B, int m) 
 
 Csr csr_multiply(const Csr &A, const Csr &B) { return multiply(A, B); }
 
+bool block_parts_complete(const Csr &A, const Csr &M, const Csr &L) {
+    const int n = M.n;
+    if (A.n != 4 * n || L.n != n) return false;
+    auto entry = [](const Csr &B, int i, int j, double *v) {
+        const int *b = B.col.data() + B.ptr[i], *e = B.col.data() + B.ptr[i + 1];
+        const int *at = std::lower_bound(b, e, j);
+        if (at == e || *at != j) return false;
+        *v = B.val[at - B.col.data()];
+        return true;
+    };
+    bool complete = true;
+#pragma omp parallel for schedule(static) reduction(&& : complete)
+    for (int r = 0; r < A.n; ++r) {
+        const int br = r / n, i = r % n;
+        double scale = 0.0;
+        int coupled = 0, own = 0;   // entries of a u row
+        for (int q = A.ptr[r]; q < A.ptr[r + 1]; ++q) scale = std::max(scale, std::fabs(A.val[q]));
+        for (int q = A.ptr[r]; q < A.ptr[r + 1]; ++q) {
+            const int bc = A.col[q] / n, j = A.col[q] % n;
+            double v = 0.0;
+            bool ok;
+            if (br < 2) {          // w rows: the w columns, and u2 in w2's
+                ok = (bc < 2 || (br == 1 && bc == 3)) && entry(M, i, j, &v);
+            } else if (bc < 2) {   // u rows: M in their layer's w columns, -L in their own
+                ok = bc == br - 2 && entry(M, i, j, &v) && std::fabs(A.val[q] - v) <= 1e-13 * scale;
+                ++coupled;
+            } else {
+                ok = bc == br && entry(L, i, j, &v) && std::fabs(A.val[q] + v) <= 1e-13 * scale;
+                ++own;
+            }
+            complete = complete && ok;
+        }
+        if (br >= 2) complete = complete && coupled == M.ptr[i + 1] - M.ptr[i] && own == L.ptr[i + 1] - L.ptr[i];
+    }
+    return complete;
+}
+
 bool build_mg_plan(const Csr &fine, const MgHierarchy &h, double omega, MgPlan &p) {
     const int nlev = (int)h.A.size();
     p = MgPlan();
