@@ -156,8 +156,9 @@ int phg_ops_mult32(phg_ops o, const char *name, float *y, const float *x, int nv
 /* Index validation (debug aid, no reference counterpart): counts the entries
  * of the handle's device index arrays outside their valid range -- the shared
  * ELL pattern, the inner / outer / p2io maps, the norm pattern, the boundary
- * column lists and the multigrid hierarchy (columns, prolongation and
- * restriction lists).  Only the indices are read.  Synchronises the stream. */
+ * column lists, the multigrid hierarchy (columns, prolongation and
+ * restriction lists, the composed operators) and the solve tables, those of
+ * the handle's time steppers among them.  Only the indices are read.  Synchronises the stream. */
 int phg_ops_validate(phg_ops o, long long *bad_entries, void *stream);
 
 /* Autotuner (no reference counterpart).  Times the candidate launch shapes

@@ -507,6 +507,14 @@ struct ColsBufs {
 }  // namespace
 
 struct phg_ops_s {
+    void add_system(const DevSolveOp *op) {
+        std::lock_guard<std::mutex> g(systems_mu);
+        systems.push_back(op);
+    }
+    void drop_system(const DevSolveOp *op) {
+        std::lock_guard<std::mutex> g(systems_mu);
+        systems.erase(std::remove(systems.begin(), systems.end(), op), systems.end());
+    }
     std::atomic<int> refs{1};   // the caller's, plus one per time stepper
     phg_mesh_s *mesh = nullptr;
     int prec = PHG_FP64;
@@ -535,6 +543,8 @@ struct phg_ops_s {
     DevEll norm;
     int restart = 30, max_iter = 20000;
     double tol = 1e-12;
+    std::mutex systems_mu;           // the time steppers' systems, for phg_ops_validate
+    std::vector<const DevSolveOp *> systems;
     int max_sms = 0;                 // SMs the persistent solver may fill (0 = all)
     long long wait_limit = 0;        // barrier wait limit of the persistent solvers (0 = default ~1 s)
     // scratch
@@ -1482,8 +1492,16 @@ extern "C" int phg_ops_validate(phg_ops o, long long *bad_entries, void *stream)
             CK(check_range(D.rf, (long long)D.Wr * nc, -1, D.n, bad, s));
         }
     }
-    for (const DevSolveOp *op : {&o->ML.op, &o->MJ.op})
-        if (op->c7) CK(check_range(op->c7, 7LL * op->A.n, 0, op->A.n, bad, s));
+    // the solve operators' own tables, and those of the handle's time steppers
+    std::lock_guard<std::mutex> g(o->systems_mu);
+    std::vector<const DevSolveOp *> solves = {&o->ML.op, &o->MJ.op};
+    solves.insert(solves.end(), o->systems.begin(), o->systems.end());
+    for (const DevSolveOp *op : solves) {
+        const int n = op->A.n;
+        if (op->A.col != o->pcol.as<int>()) CK(check_range(op->A.col, (long long)op->A.W * n, 0, n, bad, s));
+        if (op->c7) CK(check_range(op->c7, 7LL * n, 0, n, bad, s));
+        if (op->blk.c) CK(check_range(op->blk.c, (long long)MGX_WT * rs, 0, rs, bad, s));
+    }
     const MgxDev &mx = o->L.op.mgx;
     for (int l = 0; l + 1 < mx.nlev; ++l) {
         const MgxLevelDev &D = mx.lev[l];
@@ -1902,6 +1920,8 @@ struct phg_barvortex_s {
     DBuf agg;                   // solve records folded over the steps of runs since the last check
     bool agg_pending = false;
     ~phg_barvortex_s() {
+        o->drop_system(&A.op);
+        o->drop_system(&Aback.op);
         for (auto &g : graphs)
             if (g.exec) cudaGraphExecDestroy(g.exec);
     }
@@ -1932,6 +1952,7 @@ extern "C" int phg_barvortex_create(phg_ops o, const phg_bv_conf *c, const doubl
     int r;
     if ((r = build_solve_op(o, A, b->A, true))) return r;
     if ((r = build_cols(Ab, b->Ab))) return r;
+    o->add_system(&b->A.op);
     std::vector<double> lh(o->V, 0.0);
     if (coriolis) {
         if (is_device_ptr(coriolis)) CK(cudaMemcpy(lh.data(), coriolis, 8 * lh.size(), cudaMemcpyDeviceToHost));
@@ -2317,6 +2338,7 @@ int lin_backward(phg_barvortex_s *b) {
     int r;
     if ((r = build_solve_op(o, A, b->Aback, true))) return r;
     if ((r = build_cols(Ab, b->Abackb))) return r;
+    o->add_system(&b->Aback.op);
     b->have_back = true;
     return PHG_OK;
 }
@@ -2512,7 +2534,11 @@ struct phg_baroclin_s {
     std::vector<GmresStats> each;   // the last step's solve records, one per slot
     int nslots = 0;
     int *hdone = nullptr;   // pinned copy of the Picard stop flag
-    ~phg_baroclin_s() { if (hdone) cudaFreeHost(hdone); }
+    ~phg_baroclin_s() {
+        o->drop_system(&fwd.op);
+        o->drop_system(&back.op);
+        if (hdone) cudaFreeHost(hdone);
+    }
 };
 
 namespace {
@@ -2662,6 +2688,7 @@ extern "C" int phg_baroclin_create(phg_ops o, const phg_bc_conf *c, const double
     b->su = std::ldexp(1.0, (int)std::lround(std::log2(1.0 / c->tau)));
     int r;
     if ((r = build_bc_system(o, bc_params(*c, b->theta, false), b->su, b->fwd))) return r;
+    o->add_system(&b->fwd.op);
     std::vector<double> lh(o->V, 0.0);
     if (coriolis) {
         if (is_device_ptr(coriolis)) CK(cudaMemcpy(lh.data(), coriolis, 8 * lh.size(), cudaMemcpyDeviceToHost));
@@ -2782,6 +2809,7 @@ int bc_lin_dev(phg_baroclin_s *b, int kind, double *u11, double *u21, const doub
     int r, slot = 0;
     if (kind == 1 && !b->have_back) {
         if ((r = build_bc_system(o, bc_params(c, th, true), b->su, b->back))) return r;
+        o->add_system(&b->back.op);
         b->have_back = true;
     }
     const BcSystem &S = kind == 0 ? b->fwd : b->back;
