@@ -163,9 +163,9 @@ int phg_ops_validate(phg_ops o, long long *bad_entries, void *stream);
 
 /* Autotuner (no reference counterpart).  Times the candidate launch shapes
  * of the kernels a barotropic step of nmembers states runs on this handle's
- * mesh and precision -- rows per block of the persistent solver (128, 256,
- * 512, 1024) for the mass solves at nmembers and 8 x nmembers right-hand
- * sides and the Laplace solve at nmembers, the lockstep path for mass solves
+ * mesh and precision -- rows per block of the persistent solver (its own
+ * rule, 128, 256, 512, 1024) for the mass solves at nmembers and 8 x nmembers
+ * right-hand sides and the Laplace solve at nmembers, the lockstep path for mass solves
  * in mixed precision (8 or more right-hand sides), and threads per row of
  * phg_ops_mult32 at nmembers vectors -- and keeps the fastest in a
  * process-wide table consulted by every later launch of the same kernel

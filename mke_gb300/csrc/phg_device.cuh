@@ -163,7 +163,7 @@ struct GmresStats {
 
 
 // Launch shape of a solve.  rpb: rows per block of the persistent kernels
-// (no block gets fewer rows; 0 = 256).  path, for Chebyshev-solvable
+// (no block gets fewer rows; 0: no limit in mgs_kernel and chs_kernel, 256 in the others).  path, for Chebyshev-solvable
 // operators in mixed precision: 1 = lockstep launches over an interleaved
 // FP32 multi-vector (8 or more right-hand sides), 0 = per-member persistent
 // kernels, -1 = the built-in rule (by rows x right-hand sides, choose_path).

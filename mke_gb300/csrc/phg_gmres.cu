@@ -59,8 +59,8 @@ constexpr int LS_MIN_TUNED = 8;  // the fewest right-hand sides for which the au
 // block, the former win once the vectors outgrow that -- by rows x right-hand
 // sides, from about these products on (measured; see choose_path)
 constexpr long long LS_MIN_WORK = 8000000;    // Chebyshev solves
-// multigrid Laplacians (above level 5 one right-hand side's persistent solve fills
-// the chip sooner), and the fewest right-hand sides
+// multigrid Laplacians (above level 5 from more on, for time steps whose solves
+// start warm), and the fewest right-hand sides
 constexpr long long LSG_MIN_WORK = 1100000, LSG_MIN_WORK_L6 = 1500000;
 constexpr int LSG_MIN_NV = 16;
 

@@ -923,8 +923,14 @@ cudaError_t mgs_solve(const DevSolveOp &op, const MgsArgs &q, cudaStream_t s) {
     for (int l = 0; l < nlev; ++l) p.x_n[l] = x.lev[l].n;
     // Where the dense product starts.  Each sparse level costs two hand-overs
     // (about 1,500 cycles each between blocks, 150 within one); a dense product
-    // costs its multiply-adds per block, at 2 FP64 or 64 FP32 a cycle from
-    // shared memory and about 16 FP32 (4 FP64) values a cycle from L2.
+    // costs its multiply-adds per block, taken at 48 FP32 or 1.6 FP64 a cycle from
+    // shared memory and 14 or 1.5 from L2.  Against every start forced in turn
+    // (noise, to 1e-12; 1, 8, 37 and 160 right-hand sides on levels 3 to 5, 1 and 8
+    // on 6 and 7, both precisions) the choice is within 3 % of the
+    // best in 27 of 31 cases; one FP64 solve on level 3 249 us with it and 233 with
+    // the finest level dense, and one or two levels further down would be 9 to 15 %
+    // faster for 8 and 37 mixed ones on level 5 (37: 1,193 and 1,040 us) and 8 FP64
+    // ones on level 6.
     double best = 1e300;
     for (int k = x.first_dense; k < nlev; ++k)
         for (int wide = 0; wide < 2; ++wide) {
